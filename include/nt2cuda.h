@@ -468,6 +468,11 @@ nt2cuda_status nt2cuda_selftest_fold_timeout(const float* A, size_t rows, size_t
  * patterns.  Synchronous. */
 nt2cuda_status nt2cuda_selftest_x2(int which, unsigned long long* mismatches, uint32_t* first_bad,
                                    nt2cuda_stream stream);
+/* The double functors' multiply (which = 0), divide (1) and square root (2),
+ * computed on the integer pipes, against the hardware instructions over 2^30
+ * drawn operand pairs.  *mismatches = results that differ in any bit (two NaNs
+ * are equal).  Synchronous. */
+nt2cuda_status nt2cuda_selftest_f64(int which, unsigned long long* mismatches, nt2cuda_stream stream);
 
 /* --------------------------------------------------------- sigmadelta ---- */
 /* One grey video stream for the batched sigma-delta background subtraction

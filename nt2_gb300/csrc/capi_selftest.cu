@@ -2,6 +2,8 @@
 // float functors (nt2cuda/bs_x2.cuh) give the one-lane forms' bits
 // (nt2cuda/math.cuh) for every float argument (for pow: every float as
 // either argument, with drawn partners).
+// Also a check by drawn operands that the integer double multiply, divide and
+// square root (nt2cuda/f64_int.cuh) give the hardware instructions' bits.
 //
 // Each check runs one kernel over all 2^32 float bit patterns (2^31 pairs),
 // compares the packed result of both lanes with the scalar functor bit for
@@ -11,6 +13,7 @@
 #include <stdint.h>
 #include "internal.cuh"
 #include "nt2cuda/bs_x2.cuh"
+#include "nt2cuda/f64_int.cuh"
 #include "nt2cuda/launch.cuh"
 #include "nt2cuda/math.cuh"
 #include "nt2cuda/trig.cuh"
@@ -206,7 +209,77 @@ __global__ void __launch_bounds__(256) k_x2_check(int which, uint64_t pairs, x2_
   }
 }
 
+// A double from 128 drawn bits: any exponent one time in four, else one of the
+// integer forms' (512..1534) with its ends drawn often; significands random or
+// next to all zeros, all ones or one bit.
+__device__ __forceinline__ uint64_t mix64(uint64_t x)
+{
+  x += 0x9e3779b97f4a7c15ull;
+  x = (x ^ (x >> 30)) * 0xbf58476d1ce4e5b9ull;
+  x = (x ^ (x >> 27)) * 0x94d049bb133111ebull;
+  return x ^ (x >> 31);
+}
+__device__ __forceinline__ double draw_f64(uint64_t h, uint64_t g)
+{
+  const uint64_t ones = 0xfffffffffffffull, k = (g >> 8) % 52u, small = (g >> 16) & 7u;
+  uint64_t m = h & ones;
+  switch (g & 7u) {
+    case 0: m &= ~((1ull << k) - 1ull); break;
+    case 1: m |= (1ull << k) - 1ull; break;
+    case 2: m = small; break;
+    case 3: m = ones - small; break;
+    case 4: m = ((1ull << k) + small - 4ull) & ones; break;
+    default: break;
+  }
+  uint64_t e = (g >> 32) & 0x7ffu;
+  if ((g >> 44) & 3u) e = 512u + e % 1023u;
+  if (((g >> 46) & 7u) == 0u) e = ((g >> 49) & 1u ? 1532u : 510u) + ((g >> 50) & 3u);
+  return f64i::from_bits((h & 0x8000000000000000ull) | (e << 52) | m);
+}
+__device__ __forceinline__ bool same(double a, double b)
+{
+  return f64i::bits(a) == f64i::bits(b) || (a != a && b != b);
+}
+__global__ void __launch_bounds__(256) k_f64_check(int which, uint64_t draws, unsigned long long* bad)
+{
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < draws; i += (uint64_t)gridDim.x * blockDim.x) {
+    const double a = draw_f64(mix64(4 * i), mix64(4 * i + 1)), b = draw_f64(mix64(4 * i + 2), mix64(4 * i + 3));
+    bool ok;
+    if (which == 0) {
+      ok = same(f64i::mul(a, b), __dmul_rn(a, b));
+    } else if (which == 1) {
+      ok = same(f64i::div(a, b), __ddiv_rn(a, b));
+    } else {                              // the drawn value, and a rounded square
+      const double q = __dmul_rn(b, b);
+      ok = same(f64i::sqrt(a), __dsqrt_rn(a)) && same(f64i::sqrt(q), __dsqrt_rn(q));
+    }
+    if (!ok) atomicAdd(bad, 1ull);
+  }
+}
+
 }  // namespace
+
+extern "C" nt2cuda_status nt2cuda_selftest_f64(int which, unsigned long long* mismatches, nt2cuda_stream stream)
+{
+  NT2CUDA_NVTX_RANGE;
+  if (which < 0 || which > 2 || !mismatches) return NT2CUDA_ERR_ARG;
+  cudaStream_t s = as_stream(stream);
+  unsigned long long* bad = nullptr;
+  cudaError_t e = cudaMalloc(&bad, sizeof(*bad));
+  if (e != cudaSuccess) return from_cuda(e);
+  e = cudaMemsetAsync(bad, 0, sizeof(*bad), s);
+  if (e == cudaSuccess) {
+    k_f64_check<<<(unsigned)(sm_count() * 8), 256, 0, s>>>(which, (uint64_t)1 << 30, bad);
+    e = cudaGetLastError();
+  }
+  unsigned long long h = 0;
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&h, bad, sizeof(h), cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  cudaFree(bad);
+  if (e != cudaSuccess) return from_cuda(e);
+  *mismatches = h;
+  return NT2CUDA_OK;
+}
 
 extern "C" nt2cuda_status nt2cuda_selftest_x2(int which, unsigned long long* mismatches, uint32_t* first_bad,
                                               nt2cuda_stream stream)

@@ -211,7 +211,10 @@ nt2cuda_status bs_launch(const T* S, const T* K, const T* Tm, T r, T v, T* call,
     return launch_status(launch_persistent(k_blackscholes_scalar<T, CDF, P>, n, 256, waves, s, args));
   constexpr int V = 16 / (int)sizeof(T);
   size_t groups = n / V;
-  switch (unroll) {
+  // doubles: one group per thread whatever was tuned (see one_group)
+  if constexpr (sizeof(T) == 8)
+    return launch_status(launch_persistent(k_blackscholes<T, CDF, P, 1>, groups, 256, waves, s, args));
+  else switch (unroll) {
     case 1: return launch_status(launch_persistent(k_blackscholes<T, CDF, P, 1>, groups, 256, waves, s, args));
     case 4: return launch_status(launch_persistent(k_blackscholes<T, CDF, P, 4>, groups, 256, waves, s, args));
     default: return launch_status(launch_persistent(k_blackscholes<T, CDF, P, 2>, groups, 256, waves, s, args));

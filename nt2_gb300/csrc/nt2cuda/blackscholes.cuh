@@ -140,6 +140,7 @@ __global__ void __launch_bounds__(256, (kMinBlocks<T, CDF, P, U>))
       mem::store_vec<T, V>(put, i, op);
     }
   }
+  if constexpr (U > 1) {
 #pragma unroll 1
   for (; g < ngroups; g += stride) {
     T s[V], k[V], t[V], oc[V], op[V];
@@ -165,6 +166,7 @@ __global__ void __launch_bounds__(256, (kMinBlocks<T, CDF, P, U>))
     }
     mem::store_vec<T, V>(call, i, oc);
     mem::store_vec<T, V>(put, i, op);
+  }
   }
   const size_t tail0 = ngroups * V;
   if (tid < n - tail0) {

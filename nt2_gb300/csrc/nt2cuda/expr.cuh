@@ -530,6 +530,16 @@ template <> struct prog_heavy<prog<>> { static constexpr int value = 0; };
 template <class T, class E, class... As> struct prog_heavy<prog<assign<T, E>, As...>> {
   static constexpr int value = heavy_nodes<E>::value + prog_heavy<prog<As...>>::value;
 };
+// Statements with a long functor over doubles run one group per thread only:
+// they are bound by the double pipe, which two lanes a thread and a full SM of
+// threads keep busy, and each further group repeats the functor's code (one
+// exact Black-Scholes option is some 3000 instructions).
+template <class P> struct prog_f64;
+template <> struct prog_f64<prog<>> { static constexpr bool value = false; };
+template <class T, class E, class... As> struct prog_f64<prog<assign<T, E>, As...>> {
+  static constexpr bool value = std::is_same<typename value_of<E>::type, double>::value || prog_f64<prog<As...>>::value;
+};
+template <class P> struct one_group { static constexpr bool value = prog_f64<P>::value && prog_heavy<P>::value >= 1; };
 template <class P> struct base_lanes {
   static constexpr int m = prog_min_elem<P>::value;
   static constexpr int value = m >= 16 ? 1 : 16 / m;
@@ -596,11 +606,13 @@ __global__ void __launch_bounds__(256, transform_min_blocks<U>::value) k_transfo
 #pragma unroll
     for (int u = 0; u < U; ++u) r[u].template compute_store<F>(p, (g + (size_t)u * T) * V);
   }
+  if constexpr (U > 1) {
 #pragma unroll 1
-  for (; g < ngroups; g += T) {
-    pregs<P, V> r;
-    r.template load<true>(p, g * V);
-    r.template compute_store<F>(p, g * V);
+    for (; g < ngroups; g += T) {
+      pregs<P, V> r;
+      r.template load<true>(p, g * V);
+      r.template compute_store<F>(p, g * V);
+    }
   }
   const size_t tail0 = ngroups * V;
   if (tid < n - tail0) {

@@ -1,0 +1,280 @@
+// nt2cuda/f64_int.cuh -- correctly rounded double multiply, divide and square
+// root on the 32-bit integer pipes.
+//
+// GB300 executes 2 double-precision operations per clock and SM (measured 1.9
+// to 2.05 for add, multiply, fma, compare, rint and the conversions alike; 0.24
+// divisions and 0.23 roots), against 64 to 128 integer ones, so one double
+// instruction holds its pipe as long as 32 to 64 integer instructions take.  In
+// dependent chains the multiply below reaches 2.6 per clock and SM, the
+// division 1.1 and the root 1.1, and they run beside the additions, which stay
+// on the double pipe: multiply and add together 1.85 per clock against 0.95
+// for the two instructions.  2^24 exact Black-Scholes options in double went
+// from 12.35 to 6.47 ms, sin over 3000001 doubles from 256 to 159 us.
+//
+// Results are the IEEE round-to-nearest-even ones, bit for bit.  The integer
+// form covers operands whose exponents keep every intermediate normal; the
+// rest (zeros, subnormals, infinities, NaNs, results near overflow or
+// underflow) take the hardware instruction.
+//
+// The header also compiles as host C++ (without the hardware fallbacks being
+// reached through CUDA intrinsics), which is how the CPU tests check it.
+#pragma once
+#include <stdint.h>
+#if defined(__CUDACC__)
+#include <cuda_runtime.h>
+#define NT2_F64I __host__ __device__ __forceinline__
+#else
+#include <math.h>
+#include <string.h>
+#define NT2_F64I inline
+#endif
+
+namespace nt2cuda {
+namespace f64i {
+
+// --------------------------------------------------------------- words
+NT2_F64I uint64_t bits(double a)
+{
+#if defined(__CUDA_ARCH__)
+  return (uint64_t)__double_as_longlong(a);
+#else
+  uint64_t u;
+  memcpy(&u, &a, 8);
+  return u;
+#endif
+}
+NT2_F64I double from_bits(uint64_t u)
+{
+#if defined(__CUDA_ARCH__)
+  return __longlong_as_double((long long)u);
+#else
+  double a;
+  memcpy(&a, &u, 8);
+  return a;
+#endif
+}
+NT2_F64I uint32_t hi32(uint64_t u) { return (uint32_t)(u >> 32); }
+NT2_F64I uint32_t lo32(uint64_t u) { return (uint32_t)u; }
+NT2_F64I uint64_t pack(uint32_t lo, uint32_t hi) { return ((uint64_t)hi << 32) | lo; }
+// upper word of (hi:lo) << s, and lower word of (hi:lo) >> s, 0 <= s < 32
+NT2_F64I uint32_t shl_hi(uint32_t lo, uint32_t hi, uint32_t s)
+{
+#if defined(__CUDA_ARCH__)
+  return __funnelshift_l(lo, hi, s);
+#else
+  return hi32(pack(lo, hi) << s);
+#endif
+}
+NT2_F64I uint32_t shr_lo(uint32_t lo, uint32_t hi, uint32_t s)
+{
+#if defined(__CUDA_ARCH__)
+  return __funnelshift_r(lo, hi, s);
+#else
+  return lo32(pack(lo, hi) >> s);
+#endif
+}
+NT2_F64I uint32_t mulhi(uint32_t a, uint32_t b)
+{
+#if defined(__CUDA_ARCH__)
+  return __umulhi(a, b);
+#else
+  return hi32((uint64_t)a * b);
+#endif
+}
+NT2_F64I uint64_t wide(uint32_t a, uint32_t b) { return (uint64_t)a * b; }
+
+// The hardware operations (operands outside the integer forms' range).
+NT2_F64I double hw_mul(double a, double b)
+{
+#if defined(__CUDA_ARCH__)
+  return __dmul_rn(a, b);
+#else
+  return a * b;
+#endif
+}
+#if defined(__CUDACC__)
+// out of line: rarely taken, and their code would crowd the instruction cache
+static __device__ __noinline__ double cold_div(double a, double b) { return __ddiv_rn(a, b); }
+static __device__ __noinline__ double cold_sqrt(double a) { return __dsqrt_rn(a); }
+#endif
+NT2_F64I double hw_div(double a, double b)
+{
+#if defined(__CUDA_ARCH__)
+  return cold_div(a, b);
+#else
+  return a / b;
+#endif
+}
+NT2_F64I double hw_sqrt(double a)
+{
+#if defined(__CUDA_ARCH__)
+  return cold_sqrt(a);
+#else
+  return ::sqrt(a);
+#endif
+}
+// Single-precision reciprocal of x in [1, 2) and reciprocal square root of x in
+// [1, 4), with relative errors of at most 2^-23 and 2^-22.9 (the PTX ISA's
+// bounds).  They only seed the quotient and the root below.
+#if !defined(__CUDACC__)
+inline int& seed_skew() { static int s = 0; return s; }   // host tests: seeds off by this many units in the last place
+#endif
+NT2_F64I uint32_t rcp_bits(uint32_t x)
+{
+#if defined(__CUDA_ARCH__)
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(__uint_as_float(x)));
+  return __float_as_uint(r);
+#elif !defined(__CUDACC__)
+  float f;
+  memcpy(&f, &x, 4);
+  f = 1.0f / f;
+  memcpy(&x, &f, 4);
+  return x + (uint32_t)seed_skew();
+#else
+  return x;
+#endif
+}
+NT2_F64I uint32_t rsqrt_bits(uint32_t x)
+{
+#if defined(__CUDA_ARCH__)
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(__uint_as_float(x)));
+  return __float_as_uint(r);
+#elif !defined(__CUDACC__)
+  float f;
+  memcpy(&f, &x, 4);
+  f = (float)(1.0 / ::sqrt((double)f));
+  memcpy(&x, &f, 4);
+  return x + (uint32_t)seed_skew();
+#else
+  return x;
+#endif
+}
+
+// into [1/2, 1), where the bits below the exponent are the seed's significand
+NT2_F64I uint32_t seed_clamp(uint32_t r)
+{
+  r = r < 0x3f7fffffu ? r : 0x3f7fffffu;
+  return r > 0x3f000000u ? r : 0x3f000000u;
+}
+
+// Exponent fields from 512 (513) to 1534: products (quotients) of two such
+// numbers are normal.
+NT2_F64I bool mul_range(uint32_t h) { return (h & 0x7ff00000u) - 0x20000000u < 0x3ff00000u; }
+NT2_F64I bool div_range(uint32_t h) { return (h & 0x7ff00000u) - 0x20100000u < 0x3fe00000u; }
+
+// ------------------------------------------------------------ multiply
+// The 106-bit product of the 53-bit significands from four 32x32 products,
+// its leading bit at 104 or 105; shifted so that it stands at bit 52 of
+// (r1:r0) with the bits below in `rest`, of which only the top word and
+// whether anything is left matter for rounding to nearest even.  Signs and
+// exponents add up in the high word: the exponents' sum less the bias fits its
+// 11 bits, so the sign bits add without a carry into or out of them.
+NT2_F64I double mul_int(double a, double b)
+{
+  const uint64_t ua = bits(a), ub = bits(b);
+  const uint32_t ah = hi32(ua), al = lo32(ua), bh = hi32(ub), bl = lo32(ub);
+  const uint32_t xh = (ah & 0xfffffu) | 0x100000u, yh = (bh & 0xfffffu) | 0x100000u;
+  const uint64_t p0 = wide(al, bl);
+  const uint64_t mid = wide(al, yh) + (wide(xh, bl) + hi32(p0));
+  const uint64_t top = wide(xh, yh) + hi32(mid);
+  const uint32_t th = hi32(top), d = th >> 9;                      // product >= 2
+  const uint32_t s = 12u - d;
+  const uint32_t r1 = shl_hi(lo32(top), th, s), r0 = shl_hi(lo32(mid), lo32(top), s);
+  uint32_t rest = shl_hi(lo32(p0), lo32(mid), s);
+  rest |= lo32(p0) ? 1u : 0u;    // bits of p0 that were shifted into `rest` leave it off the half either way
+  uint32_t e = (ah & 0xfff00000u) + (bh & 0xfff00000u) - 0x40000000u;   // (1023 + 1) << 20: r1 holds the leading one
+  e += d << 20;
+  // + carry of rest + 0x7fffffff + (r0 & 1): past the half, or on it with r0 odd
+  const uint64_t c = (uint64_t)rest + (0x7fffffffu + (r0 & 1u));
+  return from_bits(pack(r0, r1 + e) + hi32(c));
+}
+NT2_F64I double mul(double a, double b)
+{
+  const uint32_t ah = hi32(bits(a)), bh = hi32(bits(b));
+  if (mul_range(ah) && mul_range(bh)) return mul_int(a, b);
+  return hw_mul(a, b);
+}
+
+// -------------------------------------------------------------- divide
+// With significands A and B, A doubled if A < B, so that q = A/B is in [1, 2),
+// and b = B/2^52:
+//   r1  2^32/b less at most 3: the seed R0 and one Newton step (the truncated b
+//       makes it at most 2 too large before the 2 taken off);
+//   q1  q 2^30 less at most 5, from r1 times the top 32 bits of A;
+//   q2  floor(2^23 rem1/B) or one less, rem1 = A 2^30 - q1 B < 5 B, the same way;
+// and rem2 = rem1 2^23 - q2 B says which, so that Q = q1 2^23 + q2 =
+// floor(q 2^53) exactly.  A quotient of 53-bit numbers never lies half way
+// between two of them, so (Q + 1) >> 1 is q rounded to nearest.
+NT2_F64I double div_int(double a, double b)
+{
+  const uint64_t ua = bits(a), ub = bits(b);
+  const uint32_t ah = hi32(ua), bh = hi32(ub), bl = lo32(ub);
+  const uint32_t yh = (bh & 0xfffffu) | 0x100000u;
+  const uint64_t A0 = pack(lo32(ua), (ah & 0xfffffu) | 0x100000u), B = pack(bl, yh);
+  uint32_t r = rcp_bits((shl_hi(bl, bh, 3) & 0x7fffffu) | 0x3f800000u);
+  r = seed_clamp(r);
+  const uint32_t R0 = (r & 0x7fffffu) | 0x800000u;                 // 2^24/b
+  const uint64_t P = wide(R0, shl_hi(bl, yh, 11));                 // R0 b 2^31
+  const int32_t err = -(int32_t)shr_lo(lo32(P), hi32(P), 2);       // (1 - R0 b 2^-24) 2^53, below 1.5 2^30
+  const uint32_t r1 = (R0 << 8) + (uint32_t)(int32_t)(((int64_t)(int32_t)(R0 << 7) * err) >> 52) - 2u;
+  const uint32_t d = A0 < B ? 1u : 0u;
+  const uint64_t A = A0 << d;
+  const uint32_t q1 = mulhi((uint32_t)(A >> 22), r1);
+  const uint64_t rem1 = (A << 30) - (uint64_t)q1 * B;              // in [0, 5 B); the products wrap, it does not
+  uint32_t q2 = mulhi((uint32_t)(rem1 >> 24), r1) >> 5;
+  const uint64_t rem2 = (rem1 << 23) - (uint64_t)q2 * B;           // in [0, 2 B)
+  q2 += rem2 >= B ? 2u : 1u;                                       // the one missing, and 1 to round
+  const uint64_t m = (((uint64_t)q1 << 23) + q2) >> 1;
+  const uint32_t e = (ah & 0xfff00000u) - (bh & 0xfff00000u) + 0x3fe00000u - (d << 20);   // m holds the leading one
+  return from_bits(m + pack(0u, e));
+}
+NT2_F64I double div(double a, double b)
+{
+  const uint32_t ah = hi32(bits(a)), bh = hi32(bits(b));
+  if (div_range(ah) && div_range(bh)) return div_int(a, b);
+  return hw_div(a, b);
+}
+
+// --------------------------------------------------------- square root
+// a = A 2^-52 4^k with A 2^-52 =: f in [1, 4):
+//   y1  2^32/sqrt(f) less at most 7: the seed Y0 and one Newton step;
+//   s1  sqrt(f) 2^30 less at most 9;
+//   s2  2^23 rem1/(2 sqrt(f) 2^30), rem1 = A 2^8 - s1^2, at most 2 short of
+//       what is missing;
+// Q = s1 2^23 + s2 is floor(sqrt(f) 2^53) or one less, and A 2^54 - Q^2 (which
+// fits 64 bits though its terms wrap) says which.  A root of a 53-bit number
+// never lies half way between two of them, so (Q + 1) >> 1 rounds to nearest.
+NT2_F64I double sqrt_int(double a)
+{
+  const uint64_t ua = bits(a);
+  const uint32_t ah = hi32(ua), al = lo32(ua);
+  const uint32_t odd = ((ah >> 20) & 1u) ^ 1u;
+  const uint64_t A = pack(al, (ah & 0xfffffu) | 0x100000u) << odd;
+  uint32_t r = rsqrt_bits(((shl_hi(al, ah, 3) & 0x7fffffu) | 0x3f800000u) + (odd << 23));
+  r = seed_clamp(r);
+  const uint32_t Y0 = (r & 0x7fffffu) | 0x800000u;                  // 2^24/sqrt(f)
+  const uint32_t a32 = (uint32_t)(A >> 22);                         // f 2^30
+  const uint32_t g = (uint32_t)(wide(a32, Y0) >> 24);               // sqrt(f) 2^30
+  const uint64_t G = wide(g, Y0);                                   // f Y0^2 2^-48 2^54
+  const int32_t err = -(int32_t)shr_lo(lo32(G), hi32(G), 2);        // (1 - f Y0^2 2^-48) 2^52, below 2^31
+  const uint32_t y1 = (Y0 << 8) + (uint32_t)(int32_t)(((int64_t)(int32_t)(Y0 << 7) * err) >> 52) - 5u;
+  const uint32_t s1 = mulhi(a32, y1);
+  const uint64_t rem1 = (A << 8) - wide(s1, s1);                    // below 2^35
+  const uint32_t s2 = mulhi((uint32_t)(rem1 >> 3), y1) >> 5;
+  uint64_t Q = ((uint64_t)s1 << 23) + s2;
+  const uint64_t rem2 = (A << 54) - Q * Q;                          // (T - Q)(T + Q), T = sqrt(f) 2^53
+  Q += rem2 > 2u * Q ? 2u : 1u;
+  const uint32_t e = ((ah >> 20) - odd + 1021u) >> 1;               // Q >> 1 holds the leading one
+  return from_bits((Q >> 1) + pack(0u, e << 20));
+}
+NT2_F64I double sqrt(double a)
+{
+  const uint32_t ah = hi32(bits(a));
+  if (ah - 0x20000000u < 0x3ff00000u) return sqrt_int(a);           // positive, exponent field 512 to 1534
+  return hw_sqrt(a);
+}
+
+}  // namespace f64i
+}  // namespace nt2cuda

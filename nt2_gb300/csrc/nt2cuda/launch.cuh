@@ -158,7 +158,8 @@ inline cudaError_t transform(const P& p, size_t n, cudaStream_t s, const char* t
   const bool vec = all_aligned(p, 16u);
   if (!vec) return launch_persistent(k_transform<F, 1, 1, P>, n, 256, W, s, args);
   const size_t groups = n / V;
-  switch (U) {
+  if constexpr (one_group<P>::value) return launch_persistent(k_transform<F, V, 1, P>, groups, 256, W, s, args);
+  else switch (U) {
     case 1: return launch_persistent(k_transform<F, V, 1, P>, groups, 256, W, s, args);
     case 4: return launch_persistent(k_transform<F, V, 4, P>, groups, 256, W, s, args);
     default: return launch_persistent(k_transform<F, V, 2, P>, groups, 256, W, s, args);

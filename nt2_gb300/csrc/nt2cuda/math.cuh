@@ -14,6 +14,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include "f64_int.cuh"
 
 namespace nt2cuda {
 namespace math {
@@ -26,9 +27,9 @@ __device__ __forceinline__ float div(float a, float b) { return __fdiv_rn(a, b);
 __device__ __forceinline__ float sqrt_(float a) { return __fsqrt_rn(a); }
 __device__ __forceinline__ double add(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ double sub(double a, double b) { return __dsub_rn(a, b); }
-__device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
-__device__ __forceinline__ double div(double a, double b) { return __ddiv_rn(a, b); }
-__device__ __forceinline__ double sqrt_(double a) { return __dsqrt_rn(a); }
+__device__ __forceinline__ double mul(double a, double b) { return f64i::mul(a, b); }
+__device__ __forceinline__ double div(double a, double b) { return f64i::div(a, b); }
+__device__ __forceinline__ double sqrt_(double a) { return f64i::sqrt(a); }
 
 // NT2 fma(a,b,c) = a*b+c ; fnms(a,b,c) = c-a*b
 template <bool F> __device__ __forceinline__ float madd(float a, float b, float c)
@@ -36,9 +37,9 @@ template <bool F> __device__ __forceinline__ float madd(float a, float b, float 
 template <bool F> __device__ __forceinline__ float nmsub(float a, float b, float c)
 { return F ? __fmaf_rn(-a, b, c) : __fsub_rn(c, __fmul_rn(a, b)); }
 template <bool F> __device__ __forceinline__ double madd(double a, double b, double c)
-{ return F ? __fma_rn(a, b, c) : __dadd_rn(__dmul_rn(a, b), c); }
+{ return F ? __fma_rn(a, b, c) : __dadd_rn(mul(a, b), c); }
 template <bool F> __device__ __forceinline__ double nmsub(double a, double b, double c)
-{ return F ? __fma_rn(-a, b, c) : __dsub_rn(c, __dmul_rn(a, b)); }
+{ return F ? __fma_rn(-a, b, c) : __dsub_rn(c, mul(a, b)); }
 
 __device__ __forceinline__ float fbits(uint32_t u) { return __uint_as_float(u); }
 __device__ __forceinline__ double dbits(uint64_t u) { return __longlong_as_double((long long)u); }

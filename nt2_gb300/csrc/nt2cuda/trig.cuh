@@ -241,10 +241,10 @@ __device__ __forceinline__ int cephes(float x, float& xr)
 }
 __device__ __forceinline__ int cephes(double x, double& xr)
 {
-  const double xi = rint(__dmul_rn(x, dbits(td::twoopi)));
-  double r = __dsub_rn(x, __dmul_rn(xi, dbits(td::pio2_1)));
-  r = __dsub_rn(r, __dmul_rn(xi, dbits(td::pio2_2)));
-  xr = __dsub_rn(r, __dmul_rn(xi, dbits(td::pio2_3)));
+  const double xi = rint(math::mul(x, dbits(td::twoopi)));
+  double r = __dsub_rn(x, math::mul(xi, dbits(td::pio2_1)));
+  r = __dsub_rn(r, math::mul(xi, dbits(td::pio2_2)));
+  xr = __dsub_rn(r, math::mul(xi, dbits(td::pio2_3)));
   return (int)xi & 3;     // |xi| <= 40 (or NaN, whose xr is NaN whatever n is)
 }
 template <class T, class C> __device__ __forceinline__ int medium_impl(T t, T& xr, T invpio2, T p1, T p2, T p2t, T p3, T p3t)
@@ -482,8 +482,8 @@ __device__ __forceinline__ int reduce_pi(float x, float& xr, bool)
 }
 __device__ __forceinline__ int reduce_pi(double x, double& xr, bool simd)
 {
-  const double xi = rint(__dmul_rn(x, 2.0));
-  xr = __dmul_rn(__dsub_rn(x, __dmul_rn(xi, 0.5)), dbits(td::pi));
+  const double xi = rint(math::mul(x, 2.0));
+  xr = math::mul(__dsub_rn(x, math::mul(xi, 0.5)), dbits(td::pi));
   // SSE2 converts packed doubles through int32 (cvttpd2dq); scalar code casts to int64
   return simd ? (toint32(xi) & 3) : (int)(toint64(xi) & 3);
 }
@@ -499,8 +499,8 @@ __device__ __forceinline__ int reduce_deg(float x, float& xr, bool)
 }
 __device__ __forceinline__ int reduce_deg(double x, double& xr, bool simd)
 {
-  const double xi = rint(__dmul_rn(x, dbits(0x3f86c16c16c16c17ull)));
-  xr = __dmul_rn(__dsub_rn(x, __dmul_rn(xi, 90.0)), dbits(0x3f91df46a2529d39ull));
+  const double xi = rint(math::mul(x, dbits(0x3f86c16c16c16c17ull)));
+  xr = math::mul(__dsub_rn(x, math::mul(xi, 90.0)), dbits(0x3f91df46a2529d39ull));
   return simd ? (toint32(xi) & 3) : (int)(toint64(xi) & 3);
 }
 template <int K, class T> __device__ __forceinline__ int reduce_unit(T x, T& xr, bool simd)
@@ -540,16 +540,16 @@ template <bool F> __device__ __forceinline__ double sin_eval(double z, double x)
 {
   constexpr uint64_t C[6] = {0x3de5d8fd1fcf0ec1ull, 0xbe5ae5e5a9291691ull, 0x3ec71de3567d4896ull,
                              0xbf2a01a019bfdf03ull, 0x3f8111111110f7d0ull, 0xbfc5555555555548ull};
-  return math::madd<F>(__dmul_rn(math::horner<F>(z, C), z), x, x);
+  return math::madd<F>(math::mul(math::horner<F>(z, C), z), x, x);
 }
 template <bool F> __device__ __forceinline__ double tan_eval(double x)
 {
   constexpr uint64_t N[3] = {0xc0c992d8d24f3f38ull, 0x413199eca5fc9dddull, 0xc1711fead3299176ull};
   constexpr uint64_t D[5] = {0x3ff0000000000000ull, 0x40cab8a5eeb36572ull, 0xc13427bc582abc96ull,
                              0x4177d98fc2ead8efull, 0xc189afe03cbe5a31ull};
-  const double zz = __dmul_rn(x, x);
-  const double q = __ddiv_rn(math::horner<F>(zz, N), math::horner<F>(zz, D));
-  return math::madd<F>(x, __dmul_rn(zz, q), x);
+  const double zz = math::mul(x, x);
+  const double q = math::div(math::horner<F>(zz, N), math::horner<F>(zz, D));
+  return math::madd<F>(x, math::mul(zz, q), x);
 }
 
 template <class T> __device__ __forceinline__ T oneo_180();
@@ -786,15 +786,15 @@ template <bool F> __device__ __forceinline__ double asin(double a0)
     r = x;
   } else if (x > 0.625) {
     double zz1 = __dsub_rn(1.0, x);
-    const double vp = __ddiv_rn(__dmul_rn(zz1, math::horner<F>(zz1, P1)), math::horner<F>(zz1, Q1));
-    zz1 = __dsqrt_rn(__dadd_rn(zz1, zz1));
+    const double vp = math::div(math::mul(zz1, math::horner<F>(zz1, P1)), math::horner<F>(zz1, Q1));
+    zz1 = math::sqrt_(__dadd_rn(zz1, zz1));
     double z = __dsub_rn(dbits(td::pio4), zz1);
-    zz1 = F ? __fma_rn(zz1, vp, -dbits(tdi::pio2lo)) : __dsub_rn(__dmul_rn(zz1, vp), dbits(tdi::pio2lo));
+    zz1 = F ? __fma_rn(zz1, vp, -dbits(tdi::pio2lo)) : __dsub_rn(math::mul(zz1, vp), dbits(tdi::pio2lo));
     z = __dsub_rn(z, zz1);
     r = __dadd_rn(z, dbits(td::pio4));
   } else {
-    const double zz2 = __dmul_rn(a0, a0);
-    const double z = __ddiv_rn(__dmul_rn(zz2, math::horner<F>(zz2, P2)), math::horner<F>(zz2, Q2));
+    const double zz2 = math::mul(a0, a0);
+    const double z = math::div(math::mul(zz2, math::horner<F>(zz2, P2)), math::horner<F>(zz2, Q2));
     r = math::madd<F>(x, z, x);
   }
   if (x > 1.0) return __longlong_as_double(0x7ff8000000000000ll);
@@ -804,7 +804,7 @@ template <bool F> __device__ __forceinline__ double acos(double a0)
 {
   double x = fabs(a0);
   const bool larger = x > 0.5;
-  x = larger ? __dsqrt_rn(math::madd<F>(-0.5, x, 0.5)) : a0;
+  x = larger ? math::sqrt_(math::madd<F>(-0.5, x, 0.5)) : a0;
   x = asin<F>(x);
   x = __dadd_rn(x, larger ? x : 0.0);
   x = (a0 < -0.5) ? __dsub_rn(dbits(td::pi), x) : x;
@@ -822,10 +822,10 @@ template <bool F> __device__ __forceinline__ double kernel_atan(double a0)
   const bool flag2 = flag1 && x >= dbits(tdi::tanpio8);
   double yy = flag1 ? 0.0 : dbits(td::pio2);
   yy = flag2 ? dbits(td::pio4) : yy;
-  double xx = flag1 ? x : -__ddiv_rn(1.0, x);
-  xx = flag2 ? __ddiv_rn(__dsub_rn(x, 1.0), __dadd_rn(x, 1.0)) : xx;
-  double z = __dmul_rn(xx, xx);
-  z = __ddiv_rn(__dmul_rn(z, math::horner<F>(z, P)), math::horner<F>(z, Q));
+  double xx = flag1 ? x : -math::div(1.0, x);
+  xx = flag2 ? math::div(__dsub_rn(x, 1.0), __dadd_rn(x, 1.0)) : xx;
+  double z = math::mul(xx, xx);
+  z = math::div(math::mul(z, math::horner<F>(z, P)), math::horner<F>(z, Q));
   z = math::madd<F>(xx, z, xx);
   z = __dadd_rn(z, flag2 ? dbits(tdi::pio4lo) : 0.0);
   z = __dadd_rn(z, flag1 ? 0.0 : dbits(tdi::pio2lo));
