@@ -276,5 +276,46 @@ NT2_F64I double sqrt(double a)
   return hw_sqrt(a);
 }
 
+// ------------------------------------------------- small conversions
+// (double)k for |k| < 2^22: the float of k (exact) with its exponent rebiased.
+NT2_F64I double small_int(int k)
+{
+#if defined(__CUDA_ARCH__)
+  const uint32_t f = __float_as_uint(__int_as_float(0x4b400000 + k) - 12582912.0f);
+#else
+  const float v = (float)k;
+  uint32_t f;
+  memcpy(&f, &v, 4);
+#endif
+  const uint32_t h = ((uint32_t)((int32_t)f >> 3) & 0x8fffffffu) + 0x38000000u;
+  return from_bits(pack(f << 29, k ? h : 0u));
+}
+// rint(t) as an integer and as a double, for |t| < 2^22 (unspecified beyond):
+// one addition on the double pipe, where rint and the conversion take two.
+NT2_F64I double round_small(double t, int& k)
+{
+#if defined(__CUDA_ARCH__)
+  k = (int)lo32(bits(__dadd_rn(t, 6755399441055744.0)));
+#else
+  k = (int)lo32(bits(t + 6755399441055744.0));
+#endif
+  return small_int(k);
+}
+// k*c for k = small_int(n), c a normal constant of moderate size (k = 0 is no operand of the integer multiply)
+NT2_F64I double mul_small(double k, int n, double c) { return n ? mul_int(k, c) : 0.0; }
+// x * 2^n where the caller knows x and the result to be normal
+NT2_F64I double scale(double x, int n) { return from_bits(bits(x) + pack(0u, (uint32_t)n << 20)); }
+// x / 2
+NT2_F64I double half(double x)
+{
+  if ((hi32(bits(x)) & 0x7fffffffu) - 0x00200000u < 0x7fd00000u) return scale(x, -1);
+  return hw_mul(x, 0.5);
+}
+// x < c for x >= 0 or NaN without its sign, c > 0: the bits compare as integers
+NT2_F64I bool below(double x, double c) { return bits(x) < bits(c); }
+// the high word without its sign: |x| >= 2^e and non-finite tests on the top 32 bits
+NT2_F64I uint32_t abs_hi(double x) { return hi32(bits(x)) & 0x7fffffffu; }
+NT2_F64I bool is_zero(double x) { return (bits(x) << 1) == 0ull; }
+
 }  // namespace f64i
 }  // namespace nt2cuda

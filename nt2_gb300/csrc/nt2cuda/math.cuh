@@ -59,7 +59,8 @@ __device__ __forceinline__ double horner(double x, const uint64_t (&c)[N])
 {
   double acc = dbits(c[0]);
 #pragma unroll
-  for (int i = 1; i < N; ++i) acc = madd<F>(x, acc, dbits(c[i]));
+  for (int i = 1; i < N; ++i)   // a leading 1 is a coefficient of several: x*1 is x
+    acc = (i == 1 && c[0] == 0x3ff0000000000000ull) ? add(x, dbits(c[1])) : madd<F>(x, acc, dbits(c[i]));
   return acc;
 }
 
@@ -344,6 +345,16 @@ __device__ __forceinline__ void fastnormcdf_pair(float a0, float& pos, float& ne
   neg = (-a0 > 0.0f) ? om : w;
 }
 
+// expo_base selections and the scale by 2^n in NT2's order (arguments near or past the range's ends)
+__device__ __forceinline__ double expo_select(double a0, double c, int n, double minl, double maxl)
+{
+  const unsigned long long ik = (unsigned long long)((long long)n + 1023);
+  double r = mul(c, __longlong_as_double((long long)(ik << 52)));
+  r = (a0 <= minl) ? 0.0 : r;
+  r = (a0 >= maxl) ? __longlong_as_double(0x7ff0000000000000ll) : r;
+  return (a0 != a0) ? a0 : r;
+}
+
 // --------------------------------------------------------------- double exp
 // modules/core/exponential/include/nt2/exponential/functions/scalar/impl/expo/d_expo_reduction.hpp:57-82
 // selections: .../exponential/functions/simd/common/impl/expo/expo_base.hpp:31-45
@@ -352,47 +363,60 @@ __device__ __forceinline__ double exp(double a0)
 {
   constexpr uint64_t P[5] = {0x3e66376972bea4d0ull, 0xbebbbd41c5d26bf1ull, 0x3f11566aaf25de2cull,
                              0xbf66c16c16bebd93ull, 0x3fc555555555553eull};
-  double k = rint(mul(dbits(cd::invlog_2), a0));
-  double hi = nmsub<F>(k, dbits(cd::log_2hi), a0);
-  double lo = mul(k, dbits(cd::log_2lo));
+  int n;
+  const double k = f64i::round_small(mul(dbits(cd::invlog_2), a0), n);
+  double hi = __fma_rn(-k, dbits(cd::log_2hi), a0);            // k*log_2hi is exact: 11 and 32 bits
+  double lo = f64i::mul_small(k, n, dbits(cd::log_2lo));
   double x = sub(hi, lo);
   double t = mul(x, x);
   double c = nmsub<F>(t, horner<F>(t, P), x);
   c = sub(1.0, sub(sub(lo, div(mul(x, c), sub(2.0, c))), hi));
-  unsigned long long ik = (unsigned long long)((long long)k + 1023);
-  double r = mul(c, __longlong_as_double((long long)(ik << 52)));
-  r = (a0 <= dbits(cd::minlog)) ? 0.0 : r;
-  r = (a0 >= dbits(cd::maxlog)) ? __longlong_as_double(0x7ff0000000000000ll) : r;
-  return (a0 != a0) ? a0 : r;
+  if (f64i::abs_hi(a0) < 0x40862000u) return f64i::scale(c, n);   // |a0| < 708: nothing to select, c*2^n normal
+  return expo_select(a0, c, n, dbits(cd::minlog), dbits(cd::maxlog));
 }
 
 // --------------------------------------------------------------- double log
 // modules/core/exponential/include/nt2/exponential/functions/simd/common/impl/logs/d_log.hpp:57-98, finalize :124-137
-template <bool F = false>
-__device__ __forceinline__ double log(double a0)
+// The mantissa's step, shared by log, log2 and log10: f = m - 1 with m in
+// [sqrt(1/2), sqrt(2)), the exponent n, s = f/(2+f), hfsq = f*f/2 and R.
+struct logparts_d { double f, s, hfsq, R, dk; int n; };
+template <bool F>
+__device__ __forceinline__ logparts_d log_kernel(double a0)
 {
   constexpr uint64_t T1[3] = {0x3fc39a09d078c69full, 0x3fcc71c51d8e78afull, 0x3fd999999997fa04ull};
   constexpr uint64_t T2[4] = {0x3fc2f112df3e5244ull, 0x3fc7466496cb03deull, 0x3fd2492494229359ull,
                               0x3fe5555555555593ull};
-  unsigned long long u = (unsigned long long)__double_as_longlong(a0);
-  long long k = (long long)((u & 0x7ff0000000000000ull) >> 52) - 1022;
-  double x = __longlong_as_double((long long)((u & ~0x7ff0000000000000ull) | 0x3fe0000000000000ull));
-  bool lt = dbits(cd::sqrt_2o_2) > x;
-  k = k + (lt ? -1 : 0);
-  double f = sub(add(x, lt ? x : 0.0), 1.0);
-  double dk = (double)k;
-  double s = div(f, add(2.0, f));
-  double z = mul(s, s);
-  double w = mul(z, z);
-  double t1 = mul(w, horner<F>(w, T1));
-  double t2 = mul(z, horner<F>(w, T2));
-  double R = add(t2, t1);
-  double hfsq = mul(0.5, mul(f, f));
-  double y = sub(mul(dk, dbits(cd::log_2hi)),
-                 sub(sub(hfsq, madd<F>(s, add(hfsq, R), mul(dk, dbits(cd::log_2lo)))), f));
+  logparts_d p;
+  const uint64_t u = f64i::bits(a0);
+  const uint32_t h = (f64i::hi32(u) & 0xfffffu) | 0x3fe00000u;
+  const bool lt = f64i::pack(f64i::lo32(u), h) < cd::sqrt_2o_2;   // both in [1/2, 1)
+  p.n = (int)((f64i::hi32(u) >> 20) & 0x7ffu) - 1022 - (lt ? 1 : 0);
+  p.f = sub(f64i::from_bits(f64i::pack(f64i::lo32(u), h + (lt ? 0x100000u : 0u))), 1.0);
+  p.dk = f64i::small_int(p.n);
+  p.s = div(p.f, add(2.0, p.f));
+  const double z = mul(p.s, p.s);
+  const double w = mul(z, z);
+  const double t1 = mul(w, horner<F>(w, T1));
+  const double t2 = mul(z, horner<F>(w, T2));
+  p.R = add(t2, t1);
+  p.hfsq = f64i::half(mul(p.f, p.f));
+  return p;
+}
+
+__device__ __forceinline__ double log_finalize(double a0, double y)
+{
+  if (f64i::hi32(f64i::bits(a0)) < 0x7ff00000u && !f64i::is_zero(a0)) return y;   // positive and finite
   y = (a0 < 0.0 || a0 != a0) ? __longlong_as_double(0x7fffffffffffffffll) : y;
   y = (a0 == __longlong_as_double(0x7ff0000000000000ll)) ? a0 : y;
   return (a0 == 0.0) ? __longlong_as_double((long long)0xfff0000000000000ull) : y;
+}
+
+template <bool F = false>
+__device__ __forceinline__ double log(double a0)
+{
+  const logparts_d p = log_kernel<F>(a0);
+  const double m = sub(sub(p.hfsq, madd<F>(p.s, add(p.hfsq, p.R), f64i::mul_small(p.dk, p.n, dbits(cd::log_2lo)))), p.f);
+  return log_finalize(a0, __fma_rn(p.dk, dbits(cd::log_2hi), -m));   // dk*log_2hi is exact: 11 and 32 bits
 }
 
 // ------------------------------------ double exp2, exp10, log2, log10
@@ -406,26 +430,19 @@ struct cd2 {
                             invlog_10 = 0x3fdbcb7b1526e50dull, log_2olog_10 = 0x3fd34413509f79ffull;
 };
 
-__device__ __forceinline__ double expo_select(double a0, double c, double k, double minl, double maxl)
-{
-  unsigned long long ik = (unsigned long long)((long long)k + 1023);
-  double r = mul(c, __longlong_as_double((long long)(ik << 52)));
-  r = (a0 <= minl) ? 0.0 : r;
-  r = (a0 >= maxl) ? __longlong_as_double(0x7ff0000000000000ll) : r;
-  return (a0 != a0) ? a0 : r;
-}
-
 template <bool F = false>
 __device__ __forceinline__ double exp2(double a0)
 {
   constexpr uint64_t P[5] = {0x3e66376972bea4d0ull, 0xbebbbd41c5d26bf1ull, 0x3f11566aaf25de2cull,
                              0xbf66c16c16bebd93ull, 0x3fc555555555553eull};
-  double k = rint(a0);
+  int n;
+  const double k = f64i::round_small(a0, n);
   double x = mul(sub(a0, k), dbits(cd2::log_2));
   double t = mul(x, x);
   double c = nmsub<F>(t, horner<F>(t, P), x);
   c = sub(1.0, sub(div(-mul(x, c), sub(2.0, c)), x));       // oneminus(((-(x*c)/(2-c))-x))
-  return expo_select(a0, c, k, dbits(cd2::minlog2), dbits(cd2::maxlog2));
+  if (f64i::abs_hi(a0) < 0x408fe800u) return f64i::scale(c, n);   // |a0| < 1021
+  return expo_select(a0, c, n, dbits(cd2::minlog2), dbits(cd2::maxlog2));
 }
 
 template <bool F = false>
@@ -435,59 +452,38 @@ __device__ __forceinline__ double exp10(double a0)
                              0x40a2b4798e134a01ull};
   constexpr uint64_t Q[4] = {0x3ff0000000000000ull, 0x405545fdce51ca08ull, 0x4093e05eefd67782ull,
                              0x40a03f37650df6e2ull};
-  double k = rint(mul(dbits(cd2::invlog10_2), a0));
-  double x = nmsub<F>(k, dbits(cd2::log10_2hi), a0);
-  x = nmsub<F>(k, dbits(cd2::log10_2lo), x);
+  int n;
+  const double k = f64i::round_small(mul(dbits(cd2::invlog10_2), a0), n);
+  double x = __fma_rn(-k, dbits(cd2::log10_2hi), a0);          // k*log10_2hi is exact
+  x = F ? __fma_rn(-k, dbits(cd2::log10_2lo), x) : sub(x, f64i::mul_small(k, n, dbits(cd2::log10_2lo)));
   double xx = mul(x, x);
   double px = mul(x, horner<F>(xx, P));
   double x2 = div(px, sub(horner<F>(xx, Q), px));
   double c = add(add(x2, x2), 1.0);                         // oneplus(x2+x2)
-  return expo_select(a0, c, k, dbits(cd2::minlog10), dbits(cd2::maxlog10));
+  if (f64i::abs_hi(a0) < 0x40733000u) return f64i::scale(c, n);   // |a0| < 307
+  return expo_select(a0, c, n, dbits(cd2::minlog10), dbits(cd2::maxlog10));
 }
 
 // d_log.hpp kernel_log (:57-87): returns -(hfsq - s*(hfsq+R) - f), the log of the mantissa
 template <bool F>
-__device__ __forceinline__ double log_mantissa(double a0, double& dk)
+__device__ __forceinline__ double log_mantissa(const logparts_d& p)
 {
-  constexpr uint64_t T1[3] = {0x3fc39a09d078c69full, 0x3fcc71c51d8e78afull, 0x3fd999999997fa04ull};
-  constexpr uint64_t T2[4] = {0x3fc2f112df3e5244ull, 0x3fc7466496cb03deull, 0x3fd2492494229359ull,
-                              0x3fe5555555555593ull};
-  unsigned long long u = (unsigned long long)__double_as_longlong(a0);
-  long long k = (long long)((u & 0x7ff0000000000000ull) >> 52) - 1022;
-  double x = __longlong_as_double((long long)((u & ~0x7ff0000000000000ull) | 0x3fe0000000000000ull));
-  bool lt = dbits(cd::sqrt_2o_2) > x;
-  k = k + (lt ? -1 : 0);
-  double f = sub(add(x, lt ? x : 0.0), 1.0);
-  dk = (double)k;
-  double s = div(f, add(2.0, f));
-  double z = mul(s, s);
-  double w = mul(z, z);
-  double R = add(mul(z, horner<F>(w, T2)), mul(w, horner<F>(w, T1)));
-  double hfsq = mul(0.5, mul(f, f));
-  return -sub(sub(hfsq, mul(s, add(hfsq, R))), f);
-}
-
-__device__ __forceinline__ double log_finalize(double a0, double y)
-{
-  y = (a0 < 0.0 || a0 != a0) ? __longlong_as_double(0x7fffffffffffffffll) : y;
-  y = (a0 == __longlong_as_double(0x7ff0000000000000ll)) ? a0 : y;
-  return (a0 == 0.0) ? __longlong_as_double((long long)0xfff0000000000000ull) : y;
+  return -sub(sub(p.hfsq, mul(p.s, add(p.hfsq, p.R))), p.f);
 }
 
 template <bool F = false>
 __device__ __forceinline__ double log2(double a0)
 {
-  double dk;
-  const double m = log_mantissa<F>(a0, dk);
-  return log_finalize(a0, madd<F>(m, dbits(cd::invlog_2), dk));
+  const logparts_d p = log_kernel<F>(a0);
+  return log_finalize(a0, madd<F>(log_mantissa<F>(p), dbits(cd::invlog_2), p.dk));
 }
 
 template <bool F = false>
 __device__ __forceinline__ double log10(double a0)
 {
-  double dk;
-  const double m = log_mantissa<F>(a0, dk);
-  return log_finalize(a0, madd<F>(m, dbits(cd2::invlog_10), mul(dk, dbits(cd2::log_2olog_10))));
+  const logparts_d p = log_kernel<F>(a0);
+  return log_finalize(a0, madd<F>(log_mantissa<F>(p), dbits(cd2::invlog_10),
+                                  f64i::mul_small(p.dk, p.n, dbits(cd2::log_2olog_10))));
 }
 
 // --------------------------------------------------- double expm1, log1p
@@ -496,22 +492,22 @@ __device__ __forceinline__ double expm1(double a0)
 {
   constexpr uint64_t P[6] = {0xBE8AFDB76E09C32Dull, 0x3ED0CFCA86E65239ull, 0xBF14CE199EAADBB7ull,
                              0x3F5A01A019FE5585ull, 0xBFA11111111110F4ull, 0x3ff0000000000000ull};
-  double k = rint(mul(dbits(cd::invlog_2), a0));
-  double hi = nmsub<F>(k, dbits(cd::log_2hi), a0);
-  double lo = mul(k, dbits(cd::log_2lo));
+  int n;
+  const double k = f64i::round_small(mul(dbits(cd::invlog_2), a0), n);
+  double hi = __fma_rn(-k, dbits(cd::log_2hi), a0);            // k*log_2hi is exact
+  double lo = f64i::mul_small(k, n, dbits(cd::log_2lo));
   double x = sub(hi, lo);
-  double hxs = mul(mul(x, x), 0.5);
+  double hxs = f64i::half(mul(x, x));
   double r1 = horner<F>(hxs, P);
-  double t = nmsub<F>(mul(r1, 0.5), x, 3.0);                 // Three - r1*Half*x
+  double t = nmsub<F>(f64i::half(r1), x, 3.0);               // Three - r1*Half*x
   double e = mul(hxs, div(sub(r1, t), nmsub<F>(x, t, 6.0)));
   double c = sub(sub(hi, x), lo);
   e = sub(sub(mul(x, sub(e, c)), c), hxs);
-  long long ik = (long long)k;
-  double two2mk = __longlong_as_double((long long)((unsigned long long)(1023 - ik) << 52));
-  double ct1 = sub(sub(1.0, two2mk), sub(e, x));
-  double ct2 = add(sub(x, add(e, two2mk)), 1.0);
-  double y = (k < 20.0) ? ct1 : ct2;
-  double r = mul(y, __longlong_as_double((long long)((unsigned long long)(ik + 1023) << 52)));
+  const double two2mk = f64i::from_bits((uint64_t)(int64_t)(1023 - n) << 52);
+  const double y = n < 20 ? sub(sub(1.0, two2mk), sub(e, x)) : add(sub(x, add(e, two2mk)), 1.0);
+  double r = mul(y, f64i::from_bits((uint64_t)(int64_t)(n + 1023) << 52));
+  const uint32_t h = f64i::hi32(f64i::bits(a0));
+  if (h < 0x40862000u || h - 0x80000000u < 0x40420000u) return r;   // -36 < a0 < 708
   r = (a0 > dbits(cd::maxlog)) ? __longlong_as_double(0x7ff0000000000000ll) : r;
   return (a0 < __longlong_as_double(0xc04205966f2b4f19ll)) ? -1.0 : r;   // Logeps
 }
@@ -521,53 +517,73 @@ __device__ __forceinline__ double log1p(double a0)
 {
   double u = add(1.0, a0);
   double r = log<F>(u);
-  r = (u != 0.0) ? add(r, div(sub(a0, sub(u, 1.0)), u)) : r;
-  return (u == __longlong_as_double(0x7ff0000000000000ll)) ? u : r;
+  // u = 0 takes log's -Inf; a sum without rounding error adds a zero (log(1) is +0), so it takes r too
+  const double d = sub(a0, sub(u, 1.0));
+  if (!f64i::is_zero(u) && !f64i::is_zero(d)) r = add(r, div(d, u));
+  return f64i::bits(u) == 0x7ff0000000000000ull ? u : r;
 }
 
 // -------------------------------------------------------------- double erfc
 // modules/core/euler/include/nt2/euler/functions/simd/common/erfc.hpp:46-89
 // kernels: modules/core/euler/include/nt2/euler/functions/details/erf_kernel.hpp:101-163
+// The three regions' rational functions, numerators and denominators in
+// decreasing powers from the sixth (the numerators' sixth is 0, and the first
+// region's polynomials are of degree 4).
+static __device__ const __align__(16) uint64_t kErfcD[3][14] = {
+  {0x3ff0000000000000ull, 0x3ff0000000000000ull, 0x3ff0000000000000ull, 0x3f110512d5b20332ull, 0x3f37ea4332348252ull,
+   0x3f53b7664358865aull, 0x3f8166f75999dbd1ull, 0x3fa4a59a4f02579cull, 0x3fb64536ca92ea2full, 0x3fc16500f106c0a5ull,
+   0x3fdd0a84eb1ca867ull, 0x3ff20dd750429b61ull, 0x3ff0000000000000ull, 0x0ull},
+  {0x3f7cf4cfe0aacbb4ull, 0x3f89a996639b0d00ull, 0x3fc033c113a7deeeull, 0x3fb2488a6b5cb5e5ull, 0x3fe307622fcff772ull,
+   0x3fd53dd7a67c7e9full, 0x3ff9e677c2777c3cull, 0x3fec1986509e687bull, 0x40053b1052dca8bdull, 0x3ff54dfe9b258a60ull,
+   0x4003adeae79b9708ull, 0x3feffffffbbb552bull, 0x3ff0000000000000ull, 0x0ull},
+  {0x3f971d0907ea7a92ull, 0x3fa47bd61bbb3843ull, 0x3fd1d7ab774bb837ull, 0x3fc42210f88b9d43ull, 0x3ff0cfd4cb6cde9full,
+   0x3fe29be1cff90d94ull, 0x400315ffdfd5ce91ull, 0x3ff44744306832aeull, 0x400afd487397568full, 0x3ff9fa202deb88e5ull,
+   0x400602f24bf3fdb6ull, 0x3fefff5a9e697ae2ull, 0x3ff0000000000000ull, 0x0ull}};
+
+// A warp's arguments fall in all three regions, so the regions share one
+// evaluation: the lane's coefficients come from its row of kErfcD (through the
+// L1), the first region's shorter polynomials start where theirs begin.
 template <bool F = false>
 __device__ __forceinline__ double erfc_abs(double x)
 {
-  constexpr uint64_t E1P[5] = {0x3f110512d5b20332ull, 0x3f53b7664358865aull, 0x3fa4a59a4f02579cull,
-                               0x3fc16500f106c0a5ull, 0x3ff20dd750429b61ull};
-  constexpr uint64_t E1Q[5] = {0x3f37ea4332348252ull, 0x3f8166f75999dbd1ull, 0x3fb64536ca92ea2full,
-                               0x3fdd0a84eb1ca867ull, 0x3ff0000000000000ull};
-  constexpr uint64_t E2P[7] = {0x0ull, 0x3f7cf4cfe0aacbb4ull, 0x3fb2488a6b5cb5e5ull, 0x3fd53dd7a67c7e9full,
-                               0x3fec1986509e687bull, 0x3ff54dfe9b258a60ull, 0x3feffffffbbb552bull};
-  constexpr uint64_t E2Q[7] = {0x3f89a996639b0d00ull, 0x3fc033c113a7deeeull, 0x3fe307622fcff772ull,
-                               0x3ff9e677c2777c3cull, 0x40053b1052dca8bdull, 0x4003adeae79b9708ull,
-                               0x3ff0000000000000ull};
-  constexpr uint64_t E3P[7] = {0x0ull, 0x3f971d0907ea7a92ull, 0x3fc42210f88b9d43ull, 0x3fe29be1cff90d94ull,
-                               0x3ff44744306832aeull, 0x3ff9fa202deb88e5ull, 0x3fefff5a9e697ae2ull};
-  constexpr uint64_t E3Q[7] = {0x3fa47bd61bbb3843ull, 0x3fd1d7ab774bb837ull, 0x3ff0cfd4cb6cde9full,
-                               0x400315ffdfd5ce91ull, 0x400afd487397568full, 0x400602f24bf3fdb6ull,
-                               0x3ff0000000000000ull};
-  double xx = mul(x, x);
-  double r1;
-  if (x < 0.65) {
-    r1 = sub(1.0, mul(x, div(horner<F>(xx, E1P), horner<F>(xx, E1Q))));
-  } else {
-    double ex = exp<F>(-xx);
-    if (x < 2.2) r1 = mul(ex, div(horner<F>(x, E2P), horner<F>(x, E2Q)));
-    else         r1 = mul(ex, div(horner<F>(x, E3P), horner<F>(x, E3Q)));
-  }
-  return (x == __longlong_as_double(0x7ff0000000000000ll)) ? 0.0 : r1;
+  const bool small = f64i::below(x, 0.65);
+  const ulonglong2* c = reinterpret_cast<const ulonglong2*>(kErfcD[small ? 0 : (f64i::below(x, 2.2) ? 1 : 2)]);
+  const double xx = mul(x, x);
+  const double t = small ? xx : x;
+  const ulonglong2 c0 = __ldg(c), c1 = __ldg(c + 1), c2 = __ldg(c + 2), c3 = __ldg(c + 3), c4 = __ldg(c + 4),
+                   c5 = __ldg(c + 5), c6 = __ldg(c + 6);
+  // p: c0.x, then c1.y, c2.y, ...; q: c0.y, c1.x, then c2.x, c3.x, ...
+  double p = madd<F>(t, dbits(c0.x), dbits(c1.y));
+  double q = madd<F>(t, madd<F>(t, dbits(c0.y), dbits(c1.x)), dbits(c2.x));
+  p = small ? dbits(c1.y) : p;
+  q = small ? dbits(c2.x) : q;
+  p = madd<F>(t, p, dbits(c2.y));
+  q = madd<F>(t, q, dbits(c3.x));
+  p = madd<F>(t, p, dbits(c3.y));
+  q = madd<F>(t, q, dbits(c4.x));
+  p = madd<F>(t, p, dbits(c4.y));
+  q = madd<F>(t, q, dbits(c5.x));
+  p = madd<F>(t, p, dbits(c5.y));
+  q = madd<F>(t, q, dbits(c6.x));
+  double ex = x;
+  if (!small) ex = exp<F>(-xx);
+  const double m = mul(ex, div(p, q));
+  const double r1 = small ? sub(1.0, m) : m;
+  return f64i::bits(x) == 0x7ff0000000000000ull ? 0.0 : r1;
 }
 
 template <bool F = false>
 __device__ __forceinline__ double erfc(double a0)
 {
   double r1 = erfc_abs<F>(fabs(a0));
-  return (a0 < 0.0) ? sub(2.0, r1) : r1;
+  // a0 < 0 (erfc_abs is 1 at -0, and 2 - 1 is 1)
+  return f64i::hi32(f64i::bits(a0)) - 0x80000000u <= 0x7ff00000u ? sub(2.0, r1) : r1;
 }
 
 template <bool F = false>
 __device__ __forceinline__ double normcdf(double a0)
 {
-  return mul(0.5, erfc<F>(mul(-dbits(cd::sqrt_2o_2), a0)));
+  return f64i::half(erfc<F>(mul(-dbits(cd::sqrt_2o_2), a0)));
 }
 
 template <bool F = false>
@@ -576,8 +592,9 @@ __device__ __forceinline__ void normcdf_pair(double a0, double& pos, double& neg
   double y = mul(-dbits(cd::sqrt_2o_2), a0);
   double r1 = erfc_abs<F>(fabs(y));
   double two_m = sub(2.0, r1);
-  pos = mul(0.5, (y < 0.0) ? two_m : r1);
-  neg = mul(0.5, (-y < 0.0) ? two_m : r1);
+  const uint32_t h = f64i::hi32(f64i::bits(y));               // -y < 0: its sign clear (either of them is 1 at 0)
+  pos = f64i::half(h - 0x80000000u <= 0x7ff00000u ? two_m : r1);
+  neg = f64i::half(h <= 0x7ff00000u ? two_m : r1);
 }
 
 // ---------------------------------------------------- sinh, cosh, tanh
