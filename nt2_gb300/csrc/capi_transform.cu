@@ -207,18 +207,17 @@ nt2cuda_status bs_launch(const T* S, const T* K, const T* Tm, T r, T v, T* call,
   if (n == 0) return NT2CUDA_OK;
   size_t nn = n;
   void* args[] = {(void*)&S, (void*)&K, (void*)&Tm, (void*)&r, (void*)&v, (void*)&call, (void*)&put, (void*)&nn};
-  if (!(aligned16(S) && aligned16(K) && aligned16(Tm) && aligned16(call) && aligned16(put)))
-    return launch_status(launch_persistent(k_blackscholes_scalar<T, CDF, P>, n, 256, waves, s, args));
-  constexpr int V = 16 / (int)sizeof(T);
-  size_t groups = n / V;
-  // doubles: one group per thread whatever was tuned (see one_group)
-  if constexpr (sizeof(T) == 8)
-    return launch_status(launch_persistent(k_blackscholes<T, CDF, P, 1>, groups, 256, waves, s, args));
-  else switch (unroll) {
-    case 1: return launch_status(launch_persistent(k_blackscholes<T, CDF, P, 1>, groups, 256, waves, s, args));
-    case 4: return launch_status(launch_persistent(k_blackscholes<T, CDF, P, 4>, groups, 256, waves, s, args));
-    default: return launch_status(launch_persistent(k_blackscholes<T, CDF, P, 2>, groups, 256, waves, s, args));
+  const bool vec = sizeof(T) == 4 && aligned16(S) && aligned16(K) && aligned16(Tm) && aligned16(call) && aligned16(put);
+  if (!vec) return launch_status(launch_persistent(k_blackscholes_scalar<T, CDF, P>, n, 256, waves, s, args));
+  if constexpr (sizeof(T) == 4) {
+    size_t groups = n / 4;
+    switch (unroll) {
+      case 1: return launch_status(launch_persistent(k_blackscholes<T, CDF, P, 1>, groups, 256, waves, s, args));
+      case 4: return launch_status(launch_persistent(k_blackscholes<T, CDF, P, 4>, groups, 256, waves, s, args));
+      default: return launch_status(launch_persistent(k_blackscholes<T, CDF, P, 2>, groups, 256, waves, s, args));
+    }
   }
+  return NT2CUDA_ERR_ARG;
 }
 
 template <class T, int CDF>

@@ -530,16 +530,29 @@ template <> struct prog_heavy<prog<>> { static constexpr int value = 0; };
 template <class T, class E, class... As> struct prog_heavy<prog<assign<T, E>, As...>> {
   static constexpr int value = heavy_nodes<E>::value + prog_heavy<prog<As...>>::value;
 };
-// Statements with a long functor over doubles run one group per thread only:
-// they are bound by the double pipe, which two lanes a thread and a full SM of
-// threads keep busy, and each further group repeats the functor's code (one
-// exact Black-Scholes option is some 3000 instructions).
+// Statements with a long functor over doubles run one element per thread and
+// trip (128-bit packs one pack): they are bound by the double and integer
+// pipes, which a full SM of threads keeps busy, 8-byte loads are coalesced all
+// the same, and each further element repeats the functor's code, which the
+// instruction cache feels (one exact Black-Scholes option is some 3500
+// instructions; two a thread ran 2^24 in 3.57 ms, one in 3.13).
 template <class P> struct prog_f64;
 template <> struct prog_f64<prog<>> { static constexpr bool value = false; };
 template <class T, class E, class... As> struct prog_f64<prog<assign<T, E>, As...>> {
   static constexpr bool value = std::is_same<typename value_of<E>::type, double>::value || prog_f64<prog<As...>>::value;
 };
 template <class P> struct one_group { static constexpr bool value = prog_f64<P>::value && prog_heavy<P>::value >= 1; };
+template <class Tag> struct simd128_tag { static constexpr bool value = false; };
+template <class Tag> struct simd128_tag<tag::simd128_<Tag>> { static constexpr bool value = true; };
+template <class E> struct has_simd128 { static constexpr bool value = false; };
+template <class Tag, class... C> struct has_simd128<node<Tag, C...>> {
+  static constexpr bool value = simd128_tag<Tag>::value || (false || ... || has_simd128<C>::value);
+};
+template <class P> struct prog_simd128;
+template <> struct prog_simd128<prog<>> { static constexpr bool value = false; };
+template <class T, class E, class... As> struct prog_simd128<prog<assign<T, E>, As...>> {
+  static constexpr bool value = has_simd128<E>::value || prog_simd128<prog<As...>>::value;
+};
 template <class P> struct base_lanes {
   static constexpr int m = prog_min_elem<P>::value;
   static constexpr int value = m >= 16 ? 1 : 16 / m;
@@ -584,10 +597,14 @@ template <class T, class E, class... As, int V> struct pregs<prog<assign<T, E>, 
 // per thread by the first threads of the grid.
 // Unrolled variants ask the compiler for enough resident blocks that the
 // extra groups in flight are not paid for with occupancy.
-template <int U> struct transform_min_blocks { static constexpr int value = U == 1 ? 1 : (U == 2 ? 4 : 3); };
+// The one-element statements over doubles keep 64 registers, so that four
+// blocks' integer and double phases overlap.
+template <int U, class P> struct transform_min_blocks {
+  static constexpr int value = one_group<P>::value ? 4 : (U == 1 ? 1 : (U == 2 ? 4 : 3));
+};
 
 template <bool F, int V, int U, class P>
-__global__ void __launch_bounds__(256, transform_min_blocks<U>::value) k_transform(P p, size_t n)
+__global__ void __launch_bounds__(256, (transform_min_blocks<U, P>::value)) k_transform(P p, size_t n)
 {
   const size_t ngroups = n / V;
   const size_t T = (size_t)gridDim.x * blockDim.x;
@@ -614,6 +631,7 @@ __global__ void __launch_bounds__(256, transform_min_blocks<U>::value) k_transfo
       r.template compute_store<F>(p, g * V);
     }
   }
+  if constexpr (V == 1) return;
   const size_t tail0 = ngroups * V;
   if (tid < n - tail0) {
     pregs<P, 1> r;

@@ -83,34 +83,13 @@ NT2_F64I uint32_t mulhi(uint32_t a, uint32_t b)
 }
 NT2_F64I uint64_t wide(uint32_t a, uint32_t b) { return (uint64_t)a * b; }
 
-// The hardware operations (operands outside the integer forms' range).
+// The hardware multiply (operands outside the integer form's range).
 NT2_F64I double hw_mul(double a, double b)
 {
 #if defined(__CUDA_ARCH__)
   return __dmul_rn(a, b);
 #else
   return a * b;
-#endif
-}
-#if defined(__CUDACC__)
-// out of line: rarely taken, and their code would crowd the instruction cache
-static __device__ __noinline__ double cold_div(double a, double b) { return __ddiv_rn(a, b); }
-static __device__ __noinline__ double cold_sqrt(double a) { return __dsqrt_rn(a); }
-#endif
-NT2_F64I double hw_div(double a, double b)
-{
-#if defined(__CUDA_ARCH__)
-  return cold_div(a, b);
-#else
-  return a / b;
-#endif
-}
-NT2_F64I double hw_sqrt(double a)
-{
-#if defined(__CUDA_ARCH__)
-  return cold_sqrt(a);
-#else
-  return ::sqrt(a);
 #endif
 }
 // Single-precision reciprocal of x in [1, 2) and reciprocal square root of x in
@@ -164,11 +143,24 @@ NT2_F64I uint32_t seed_clamp(uint32_t r)
 NT2_F64I bool mul_range(uint32_t h) { return (h & 0x7ff00000u) - 0x20000000u < 0x3ff00000u; }
 NT2_F64I bool div_range(uint32_t h) { return (h & 0x7ff00000u) - 0x20100000u < 0x3fe00000u; }
 
+// (hi:lo) + carry of x + y
+NT2_F64I uint64_t add_carry_of(uint32_t x, uint32_t y, uint32_t lo, uint32_t hi)
+{
+#if defined(__CUDA_ARCH__)
+  asm("{\n\t.reg .u32 t;\n\tadd.cc.u32 t, %2, %3;\n\taddc.cc.u32 %0, %0, 0;\n\taddc.u32 %1, %1, 0;\n\t}"
+      : "+r"(lo), "+r"(hi)
+      : "r"(x), "r"(y));
+  return pack(lo, hi);
+#else
+  return pack(lo, hi) + hi32((uint64_t)x + y);
+#endif
+}
+
 // ------------------------------------------------------------ multiply
 // The 106-bit product of the 53-bit significands from four 32x32 products,
 // its leading bit at 104 or 105; shifted so that it stands at bit 52 of
-// (r1:r0) with the bits below in `rest`, of which only the top word and
-// whether anything is left matter for rounding to nearest even.  Signs and
+// (r1:r0) with the bits below in `rest`, of which the top word and whether
+// anything is left decide the rounding to nearest even.  Signs and
 // exponents add up in the high word: the exponents' sum less the bias fits its
 // 11 bits, so the sign bits add without a carry into or out of them.
 NT2_F64I double mul_int(double a, double b)
@@ -182,13 +174,12 @@ NT2_F64I double mul_int(double a, double b)
   const uint32_t th = hi32(top), d = th >> 9;                      // product >= 2
   const uint32_t s = 12u - d;
   const uint32_t r1 = shl_hi(lo32(top), th, s), r0 = shl_hi(lo32(mid), lo32(top), s);
-  uint32_t rest = shl_hi(lo32(p0), lo32(mid), s);
-  rest |= lo32(p0) ? 1u : 0u;    // bits of p0 that were shifted into `rest` leave it off the half either way
-  uint32_t e = (ah & 0xfff00000u) + (bh & 0xfff00000u) - 0x40000000u;   // (1023 + 1) << 20: r1 holds the leading one
-  e += d << 20;
-  // + carry of rest + 0x7fffffff + (r0 & 1): past the half, or on it with r0 odd
-  const uint64_t c = (uint64_t)rest + (0x7fffffffu + (r0 & 1u));
-  return from_bits(pack(r0, r1 + e) + hi32(c));
+  const uint32_t rest = shl_hi(lo32(p0), lo32(mid), s);
+  // past the half, or on it with r0 odd or bits of p0 left (those of them that
+  // were shifted into `rest` keep it off the half either way)
+  const uint32_t below = 0x7fffffffu + ((r0 & 1u) | (lo32(p0) < 1u ? lo32(p0) : 1u));
+  const uint32_t e = (ah & 0xfff00000u) + (bh & 0xfff00000u) - 0x40000000u;   // (1023 + 1) << 20: r1 holds the leading one
+  return from_bits(add_carry_of(rest, below, r0, r1 + e + (d << 20)));
 }
 NT2_F64I double mul(double a, double b)
 {
@@ -196,6 +187,9 @@ NT2_F64I double mul(double a, double b)
   if (mul_range(ah) && mul_range(bh)) return mul_int(a, b);
   return hw_mul(a, b);
 }
+#if defined(__CUDACC__)
+static __device__ __noinline__ double mul_any(double a, double b) { return mul(a, b); }   // for rarely run code
+#endif
 
 // -------------------------------------------------------------- divide
 // With significands A and B, A doubled if A < B, so that q = A/B is in [1, 2),
@@ -230,11 +224,23 @@ NT2_F64I double div_int(double a, double b)
   const uint32_t e = (ah & 0xfff00000u) - (bh & 0xfff00000u) + 0x3fe00000u - (d << 20);   // m holds the leading one
   return from_bits(m + pack(0u, e));
 }
+// Out of line: a functor has several, each some 55 instructions, and the
+// statements' loop bodies already exceed the instruction cache's first levels
+// (exact Black-Scholes 3.13 ms with every division inlined, 2.89 called).
+#if defined(__CUDACC__)
+static __device__ __noinline__ double div_mid(double a, double b) { return div_int(a, b); }
+static __device__ __noinline__ double div_any(double a, double b)
+{
+  return div_range(hi32(bits(a))) && div_range(hi32(bits(b))) ? div_int(a, b) : __ddiv_rn(a, b);
+}
+#endif
 NT2_F64I double div(double a, double b)
 {
-  const uint32_t ah = hi32(bits(a)), bh = hi32(bits(b));
-  if (div_range(ah) && div_range(bh)) return div_int(a, b);
-  return hw_div(a, b);
+#if defined(__CUDA_ARCH__)
+  return div_any(a, b);
+#else
+  return div_range(hi32(bits(a))) && div_range(hi32(bits(b))) ? div_int(a, b) : a / b;
+#endif
 }
 
 // --------------------------------------------------------- square root
@@ -269,11 +275,18 @@ NT2_F64I double sqrt_int(double a)
   const uint32_t e = ((ah >> 20) - odd + 1021u) >> 1;               // Q >> 1 holds the leading one
   return from_bits((Q >> 1) + pack(0u, e << 20));
 }
+// positive, exponent field 512 to 1534
+NT2_F64I bool sqrt_range(uint32_t h) { return h - 0x20000000u < 0x3ff00000u; }
+#if defined(__CUDACC__)
+static __device__ __noinline__ double sqrt_any(double a) { return sqrt_range(hi32(bits(a))) ? sqrt_int(a) : __dsqrt_rn(a); }
+#endif
 NT2_F64I double sqrt(double a)
 {
-  const uint32_t ah = hi32(bits(a));
-  if (ah - 0x20000000u < 0x3ff00000u) return sqrt_int(a);           // positive, exponent field 512 to 1534
-  return hw_sqrt(a);
+#if defined(__CUDA_ARCH__)
+  return sqrt_any(a);
+#else
+  return sqrt_range(hi32(bits(a))) ? sqrt_int(a) : ::sqrt(a);
+#endif
 }
 
 // ------------------------------------------------- small conversions

@@ -147,7 +147,7 @@ inline cudaError_t transform(const P& p, size_t n, cudaStream_t s, const char* t
   if (n == 0) return cudaSuccess;
   alias_kind ak = classify_alias(p, n);
   if (ak == alias_kind::bad) return cudaErrorInvalidValue;
-  constexpr int V = base_lanes<P>::value;
+  constexpr int V = one_group<P>::value && !prog_simd128<P>::value ? 1 : base_lanes<P>::value;
   // statements with three or more long functors: one group per thread per trip
   if (prog_heavy<P>::value >= 3 && def.unroll == tuning::params{}.unroll) def.unroll = 1;
   const tuning::params tp = tuning::lookup(tune_key, n, def);

@@ -41,6 +41,30 @@ template <bool F> __device__ __forceinline__ double madd(double a, double b, dou
 template <bool F> __device__ __forceinline__ double nmsub(double a, double b, double c)
 { return F ? __fma_rn(-a, b, c) : __dsub_rn(c, mul(a, b)); }
 
+// The double functors below are written over an arithmetic: `any` takes every
+// operand; `mid` is the integer forms without their range checks, for the
+// arguments (nearly all) whose every product, quotient and root they cover.
+// Functors test the argument's high word once and leave the rest to an
+// out-of-line `any` evaluation of the same steps.
+struct f64_any {
+  __device__ __forceinline__ static double mul(double a, double b) { return f64i::mul_any(a, b); }
+  __device__ __forceinline__ static double div(double a, double b) { return f64i::div(a, b); }
+  __device__ __forceinline__ static double half(double a) { return f64i::half(a); }
+};
+struct f64_inl {      // `any` with the multiply inlined, for functors without a `mid` form
+  __device__ __forceinline__ static double mul(double a, double b) { return f64i::mul(a, b); }
+  __device__ __forceinline__ static double div(double a, double b) { return f64i::div(a, b); }
+};
+struct f64_mid {
+  __device__ __forceinline__ static double mul(double a, double b) { return f64i::mul_int(a, b); }
+  __device__ __forceinline__ static double div(double a, double b) { return f64i::div_mid(a, b); }
+  __device__ __forceinline__ static double half(double a) { return f64i::scale(a, -1); }
+};
+template <bool F, class A> __device__ __forceinline__ double madd(double a, double b, double c)
+{ return F ? __fma_rn(a, b, c) : __dadd_rn(A::mul(a, b), c); }
+template <bool F, class A> __device__ __forceinline__ double nmsub(double a, double b, double c)
+{ return F ? __fma_rn(-a, b, c) : __dsub_rn(c, A::mul(a, b)); }
+
 __device__ __forceinline__ float fbits(uint32_t u) { return __uint_as_float(u); }
 __device__ __forceinline__ double dbits(uint64_t u) { return __longlong_as_double((long long)u); }
 
@@ -54,13 +78,13 @@ __device__ __forceinline__ float horner(float x, const uint32_t (&c)[N])
   for (int i = 1; i < N; ++i) acc = madd<F>(x, acc, fbits(c[i]));
   return acc;
 }
-template <bool F, int N>
+template <bool F, class A = f64_inl, int N>
 __device__ __forceinline__ double horner(double x, const uint64_t (&c)[N])
 {
   double acc = dbits(c[0]);
 #pragma unroll
   for (int i = 1; i < N; ++i)   // a leading 1 is a coefficient of several: x*1 is x
-    acc = (i == 1 && c[0] == 0x3ff0000000000000ull) ? add(x, dbits(c[1])) : madd<F>(x, acc, dbits(c[i]));
+    acc = (i == 1 && c[0] == 0x3ff0000000000000ull) ? add(x, dbits(c[1])) : madd<F, A>(x, acc, dbits(c[i]));
   return acc;
 }
 
@@ -358,21 +382,34 @@ __device__ __forceinline__ double expo_select(double a0, double c, int n, double
 // --------------------------------------------------------------- double exp
 // modules/core/exponential/include/nt2/exponential/functions/scalar/impl/expo/d_expo_reduction.hpp:57-82
 // selections: .../exponential/functions/simd/common/impl/expo/expo_base.hpp:31-45
-template <bool F = false>
-__device__ __forceinline__ double exp(double a0)
+template <bool F, class A>
+__device__ __forceinline__ double exp_reduced(double a0, int& n)     // exp(a0) 2^-n
 {
   constexpr uint64_t P[5] = {0x3e66376972bea4d0ull, 0xbebbbd41c5d26bf1ull, 0x3f11566aaf25de2cull,
                              0xbf66c16c16bebd93ull, 0x3fc555555555553eull};
+  const double k = f64i::round_small(A::mul(dbits(cd::invlog_2), a0), n);
+  const double hi = __fma_rn(-k, dbits(cd::log_2hi), a0);            // k*log_2hi is exact: 11 and 32 bits
+  const double lo = f64i::mul_small(k, n, dbits(cd::log_2lo));
+  const double x = sub(hi, lo);
+  const double t = A::mul(x, x);
+  const double c = nmsub<F, A>(t, horner<F, A>(t, P), x);
+  return sub(1.0, sub(sub(lo, A::div(A::mul(x, c), sub(2.0, c))), hi));
+}
+template <bool F> static __device__ __noinline__ double exp_any(double a0)
+{
   int n;
-  const double k = f64i::round_small(mul(dbits(cd::invlog_2), a0), n);
-  double hi = __fma_rn(-k, dbits(cd::log_2hi), a0);            // k*log_2hi is exact: 11 and 32 bits
-  double lo = f64i::mul_small(k, n, dbits(cd::log_2lo));
-  double x = sub(hi, lo);
-  double t = mul(x, x);
-  double c = nmsub<F>(t, horner<F>(t, P), x);
-  c = sub(1.0, sub(sub(lo, div(mul(x, c), sub(2.0, c))), hi));
-  if (f64i::abs_hi(a0) < 0x40862000u) return f64i::scale(c, n);   // |a0| < 708: nothing to select, c*2^n normal
+  const double c = exp_reduced<F, f64_any>(a0, n);
   return expo_select(a0, c, n, dbits(cd::minlog), dbits(cd::maxlog));
+}
+template <bool F = false>
+__device__ __forceinline__ double exp(double a0)
+{
+  // 2^-200 <= |a0| < 708: the reduced argument is a0 or, as no double is that
+  // close to a multiple of log(2), above 2^-90, and exp(a0) is normal
+  if (f64i::abs_hi(a0) - 0x33700000u >= 0x40862000u - 0x33700000u) return exp_any<F>(a0);
+  int n;
+  const double c = exp_reduced<F, f64_mid>(a0, n);
+  return f64i::scale(c, n);
 }
 
 // --------------------------------------------------------------- double log
@@ -380,7 +417,7 @@ __device__ __forceinline__ double exp(double a0)
 // The mantissa's step, shared by log, log2 and log10: f = m - 1 with m in
 // [sqrt(1/2), sqrt(2)), the exponent n, s = f/(2+f), hfsq = f*f/2 and R.
 struct logparts_d { double f, s, hfsq, R, dk; int n; };
-template <bool F>
+template <bool F, class A>
 __device__ __forceinline__ logparts_d log_kernel(double a0)
 {
   constexpr uint64_t T1[3] = {0x3fc39a09d078c69full, 0x3fcc71c51d8e78afull, 0x3fd999999997fa04ull};
@@ -393,30 +430,44 @@ __device__ __forceinline__ logparts_d log_kernel(double a0)
   p.n = (int)((f64i::hi32(u) >> 20) & 0x7ffu) - 1022 - (lt ? 1 : 0);
   p.f = sub(f64i::from_bits(f64i::pack(f64i::lo32(u), h + (lt ? 0x100000u : 0u))), 1.0);
   p.dk = f64i::small_int(p.n);
-  p.s = div(p.f, add(2.0, p.f));
-  const double z = mul(p.s, p.s);
-  const double w = mul(z, z);
-  const double t1 = mul(w, horner<F>(w, T1));
-  const double t2 = mul(z, horner<F>(w, T2));
+  p.s = A::div(p.f, add(2.0, p.f));
+  const double z = A::mul(p.s, p.s);
+  const double w = A::mul(z, z);
+  const double t1 = A::mul(w, horner<F, A>(w, T1));
+  const double t2 = A::mul(z, horner<F, A>(w, T2));
   p.R = add(t2, t1);
-  p.hfsq = f64i::half(mul(p.f, p.f));
+  p.hfsq = A::half(A::mul(p.f, p.f));
   return p;
+}
+// Positive, finite, normal and no power of two: f is not 0 and at least 2^-53.
+__device__ __forceinline__ bool log_mid(double a0)
+{
+  const uint64_t u = f64i::bits(a0);
+  return f64i::hi32(u) - 0x00100000u < 0x7fe00000u && ((f64i::hi32(u) << 12) | f64i::lo32(u)) != 0u;
 }
 
 __device__ __forceinline__ double log_finalize(double a0, double y)
 {
-  if (f64i::hi32(f64i::bits(a0)) < 0x7ff00000u && !f64i::is_zero(a0)) return y;   // positive and finite
   y = (a0 < 0.0 || a0 != a0) ? __longlong_as_double(0x7fffffffffffffffll) : y;
   y = (a0 == __longlong_as_double(0x7ff0000000000000ll)) ? a0 : y;
   return (a0 == 0.0) ? __longlong_as_double((long long)0xfff0000000000000ull) : y;
 }
 
+template <bool F, class A>
+__device__ __forceinline__ double log_eval(double a0)
+{
+  const logparts_d p = log_kernel<F, A>(a0);
+  const double m = sub(sub(p.hfsq, madd<F, A>(p.s, add(p.hfsq, p.R), f64i::mul_small(p.dk, p.n, dbits(cd::log_2lo)))), p.f);
+  return __fma_rn(p.dk, dbits(cd::log_2hi), -m);   // dk*log_2hi is exact: 11 and 32 bits
+}
+template <bool F> static __device__ __noinline__ double log_any(double a0)
+{
+  return log_finalize(a0, log_eval<F, f64_any>(a0));
+}
 template <bool F = false>
 __device__ __forceinline__ double log(double a0)
 {
-  const logparts_d p = log_kernel<F>(a0);
-  const double m = sub(sub(p.hfsq, madd<F>(p.s, add(p.hfsq, p.R), f64i::mul_small(p.dk, p.n, dbits(cd::log_2lo)))), p.f);
-  return log_finalize(a0, __fma_rn(p.dk, dbits(cd::log_2hi), -m));   // dk*log_2hi is exact: 11 and 32 bits
+  return log_mid(a0) ? log_eval<F, f64_mid>(a0) : log_any<F>(a0);
 }
 
 // ------------------------------------ double exp2, exp10, log2, log10
@@ -465,25 +516,35 @@ __device__ __forceinline__ double exp10(double a0)
 }
 
 // d_log.hpp kernel_log (:57-87): returns -(hfsq - s*(hfsq+R) - f), the log of the mantissa
-template <bool F>
+template <bool F, class A>
 __device__ __forceinline__ double log_mantissa(const logparts_d& p)
 {
-  return -sub(sub(p.hfsq, mul(p.s, add(p.hfsq, p.R))), p.f);
+  return -sub(sub(p.hfsq, A::mul(p.s, add(p.hfsq, p.R))), p.f);
 }
-
+template <bool F, class A>
+__device__ __forceinline__ double log2_eval(double a0)
+{
+  const logparts_d p = log_kernel<F, A>(a0);
+  return madd<F, A>(log_mantissa<F, A>(p), dbits(cd::invlog_2), p.dk);
+}
+template <bool F, class A>
+__device__ __forceinline__ double log10_eval(double a0)
+{
+  const logparts_d p = log_kernel<F, A>(a0);
+  return madd<F, A>(log_mantissa<F, A>(p), dbits(cd2::invlog_10),
+                    f64i::mul_small(p.dk, p.n, dbits(cd2::log_2olog_10)));
+}
+template <bool F> static __device__ __noinline__ double log2_any(double a0) { return log_finalize(a0, log2_eval<F, f64_any>(a0)); }
+template <bool F> static __device__ __noinline__ double log10_any(double a0) { return log_finalize(a0, log10_eval<F, f64_any>(a0)); }
 template <bool F = false>
 __device__ __forceinline__ double log2(double a0)
 {
-  const logparts_d p = log_kernel<F>(a0);
-  return log_finalize(a0, madd<F>(log_mantissa<F>(p), dbits(cd::invlog_2), p.dk));
+  return log_mid(a0) ? log2_eval<F, f64_mid>(a0) : log2_any<F>(a0);
 }
-
 template <bool F = false>
 __device__ __forceinline__ double log10(double a0)
 {
-  const logparts_d p = log_kernel<F>(a0);
-  return log_finalize(a0, madd<F>(log_mantissa<F>(p), dbits(cd2::invlog_10),
-                                  f64i::mul_small(p.dk, p.n, dbits(cd2::log_2olog_10))));
+  return log_mid(a0) ? log10_eval<F, f64_mid>(a0) : log10_any<F>(a0);
 }
 
 // --------------------------------------------------- double expm1, log1p
@@ -543,33 +604,44 @@ static __device__ const __align__(16) uint64_t kErfcD[3][14] = {
 // A warp's arguments fall in all three regions, so the regions share one
 // evaluation: the lane's coefficients come from its row of kErfcD (through the
 // L1), the first region's shorter polynomials start where theirs begin.
-template <bool F = false>
-__device__ __forceinline__ double erfc_abs(double x)
+template <bool F, class A>
+__device__ __forceinline__ double erfc_eval(double x)
 {
   const bool small = f64i::below(x, 0.65);
   const ulonglong2* c = reinterpret_cast<const ulonglong2*>(kErfcD[small ? 0 : (f64i::below(x, 2.2) ? 1 : 2)]);
-  const double xx = mul(x, x);
+  const double xx = A::mul(x, x);
   const double t = small ? xx : x;
   const ulonglong2 c0 = __ldg(c), c1 = __ldg(c + 1), c2 = __ldg(c + 2), c3 = __ldg(c + 3), c4 = __ldg(c + 4),
                    c5 = __ldg(c + 5), c6 = __ldg(c + 6);
   // p: c0.x, then c1.y, c2.y, ...; q: c0.y, c1.x, then c2.x, c3.x, ...
-  double p = madd<F>(t, dbits(c0.x), dbits(c1.y));
-  double q = madd<F>(t, madd<F>(t, dbits(c0.y), dbits(c1.x)), dbits(c2.x));
+  double p = madd<F, A>(t, dbits(c0.x), dbits(c1.y));
+  double q = madd<F, A>(t, madd<F, A>(t, dbits(c0.y), dbits(c1.x)), dbits(c2.x));
   p = small ? dbits(c1.y) : p;
   q = small ? dbits(c2.x) : q;
-  p = madd<F>(t, p, dbits(c2.y));
-  q = madd<F>(t, q, dbits(c3.x));
-  p = madd<F>(t, p, dbits(c3.y));
-  q = madd<F>(t, q, dbits(c4.x));
-  p = madd<F>(t, p, dbits(c4.y));
-  q = madd<F>(t, q, dbits(c5.x));
-  p = madd<F>(t, p, dbits(c5.y));
-  q = madd<F>(t, q, dbits(c6.x));
+  p = madd<F, A>(t, p, dbits(c2.y));
+  q = madd<F, A>(t, q, dbits(c3.x));
+  p = madd<F, A>(t, p, dbits(c3.y));
+  q = madd<F, A>(t, q, dbits(c4.x));
+  p = madd<F, A>(t, p, dbits(c4.y));
+  q = madd<F, A>(t, q, dbits(c5.x));
+  p = madd<F, A>(t, p, dbits(c5.y));
+  q = madd<F, A>(t, q, dbits(c6.x));
   double ex = x;
   if (!small) ex = exp<F>(-xx);
-  const double m = mul(ex, div(p, q));
-  const double r1 = small ? sub(1.0, m) : m;
+  const double m = A::mul(ex, A::div(p, q));
+  return small ? sub(1.0, m) : m;
+}
+template <bool F> static __device__ __noinline__ double erfc_abs_any(double x)
+{
+  const double r1 = erfc_eval<F, f64_any>(x);
   return f64i::bits(x) == 0x7ff0000000000000ull ? 0.0 : r1;
+}
+// 2^-100 <= x < 18: the polynomials (of positive coefficients) stay within
+// 2^-10 and 2^40, and exp(-x*x) above 2^-468
+template <bool F = false>
+__device__ __forceinline__ double erfc_abs(double x)
+{
+  return f64i::hi32(f64i::bits(x)) - 0x39b00000u < 0x40320000u - 0x39b00000u ? erfc_eval<F, f64_mid>(x) : erfc_abs_any<F>(x);
 }
 
 template <bool F = false>
