@@ -394,9 +394,11 @@ __device__ __forceinline__ int level(float x)
   return (x > fbits(tf::pio4)) + (x > fbits(tf::pio2)) + (x > fbits(tf::p20pi)) + (x > fbits(tf::medpi)) +
          (x > fbits(tf::dmpi));
 }
-__device__ __forceinline__ int level(double x)
+__device__ __forceinline__ int level(double x)   // x = |x|: its bits order as integers do
 {
-  return (x > dbits(td::pio4)) + (x > dbits(td::pio2)) + (x > dbits(td::p20pi)) + (x > dbits(td::medpi));
+  const uint64_t u = f64i::bits(x);
+  const int lv = (u > td::pio4) + (u > td::pio2) + (u > td::p20pi) + (u > td::medpi);
+  return u > 0x7ff0000000000000ull ? 0 : lv;
 }
 
 // Largest |x| of a pack (NaN lanes ignored, as their level is 0); level() is
@@ -482,6 +484,12 @@ __device__ __forceinline__ int reduce_pi(float x, float& xr, bool)
 }
 __device__ __forceinline__ int reduce_pi(double x, double& xr, bool simd)
 {
+  if (f64i::abs_hi(x) < 0x41300000u) {        // |x| < 2^20; xi/2 is exact
+    int k;
+    const double xi = f64i::round_small(__dadd_rn(x, x), k);
+    xr = math::mul(__fma_rn(-xi, 0.5, x), dbits(td::pi));
+    return k & 3;
+  }
   const double xi = rint(math::mul(x, 2.0));
   xr = math::mul(__dsub_rn(x, math::mul(xi, 0.5)), dbits(td::pi));
   // SSE2 converts packed doubles through int32 (cvttpd2dq); scalar code casts to int64
@@ -499,6 +507,12 @@ __device__ __forceinline__ int reduce_deg(float x, float& xr, bool)
 }
 __device__ __forceinline__ int reduce_deg(double x, double& xr, bool simd)
 {
+  if (f64i::abs_hi(x) < 0x41900000u) {        // |x| < 2^26; 90*xi is exact
+    int k;
+    const double xi = f64i::round_small(math::mul(x, dbits(0x3f86c16c16c16c17ull)), k);
+    xr = math::mul(__fma_rn(-xi, 90.0, x), dbits(0x3f91df46a2529d39ull));
+    return k & 3;
+  }
   const double xi = rint(math::mul(x, dbits(0x3f86c16c16c16c17ull)));
   xr = math::mul(__dsub_rn(x, math::mul(xi, 90.0)), dbits(0x3f91df46a2529d39ull));
   return simd ? (toint32(xi) & 3) : (int)(toint64(xi) & 3);
@@ -542,14 +556,38 @@ template <bool F> __device__ __forceinline__ double sin_eval(double z, double x)
                              0xbf2a01a019bfdf03ull, 0x3f8111111110f7d0ull, 0xbfc5555555555548ull};
   return math::madd<F>(math::mul(math::horner<F>(z, C), z), x, x);
 }
-template <bool F> __device__ __forceinline__ double tan_eval(double x)
+template <bool F, class A = math::f64_inl> __device__ __forceinline__ double tan_eval(double x)
 {
   constexpr uint64_t N[3] = {0xc0c992d8d24f3f38ull, 0x413199eca5fc9dddull, 0xc1711fead3299176ull};
   constexpr uint64_t D[5] = {0x3ff0000000000000ull, 0x40cab8a5eeb36572ull, 0xc13427bc582abc96ull,
                              0x4177d98fc2ead8efull, 0xc189afe03cbe5a31ull};
-  const double zz = math::mul(x, x);
-  const double q = math::div(math::horner<F>(zz, N), math::horner<F>(zz, D));
-  return math::madd<F>(x, math::mul(zz, q), x);
+  const double zz = A::mul(x, x);
+  const double q = A::div(math::horner<F, A>(zz, N), math::horner<F, A>(zz, D));
+  return math::madd<F, A>(x, A::mul(zz, q), x);
+}
+// sin_eval or (cosine) cos_eval of xr, z = xr*xr, without a branch: the
+// coefficients come from the lane's row of the table (through the L1), the
+// cosine's first step is taken by all and dropped by the sine's lanes.
+static __device__ const __align__(16) uint64_t kSinCosD[2][6] = {
+  {0x3de5d8fd1fcf0ec1ull, 0xbe5ae5e5a9291691ull, 0x3ec71de3567d4896ull, 0xbf2a01a019bfdf03ull, 0x3f8111111110f7d0ull,
+   0xbfc5555555555548ull},
+  {0xbe21eea7c1e514d4ull, 0x3e927e4f8e06d9a5ull, 0xbefa01a019ddbcd9ull, 0x3f56c16c16c15d47ull, 0xbfa5555555555551ull,
+   0x3fe0000000000000ull}};
+template <bool F, class A> __device__ __forceinline__ double sincos_eval(bool cosine, double xr)
+{
+  const ulonglong2* c = reinterpret_cast<const ulonglong2*>(kSinCosD[cosine ? 1 : 0]);
+  const ulonglong2 c0 = __ldg(c), c1 = __ldg(c + 1), c2 = __ldg(c + 2);
+  const double z = A::mul(xr, xr);
+  const double first = math::madd<F, A>(z, dbits(0x3da8ff831ad9b219ull), dbits(c0.x));
+  double h = cosine ? first : dbits(c0.x);
+  h = math::madd<F, A>(z, h, dbits(c0.y));
+  h = math::madd<F, A>(z, h, dbits(c1.x));
+  h = math::madd<F, A>(z, h, dbits(c1.y));
+  h = math::madd<F, A>(z, h, dbits(c2.x));
+  h = math::madd<F, A>(z, h, dbits(c2.y));
+  const double t = A::mul(h, z), w = cosine ? 1.0 : xr;
+  if constexpr (F) return __fma_rn(cosine ? -h : t, cosine ? z : xr, w);
+  return __dadd_rn(cosine ? -t : A::mul(t, xr), w);
 }
 
 template <class T> __device__ __forceinline__ T oneo_180();
@@ -585,10 +623,11 @@ template <int K, class T> __device__ __forceinline__ bool cot_invalid(T a0)
 
 // trig_base sina / cosa / tana / cota (functions/simd/common/impl/trigo/trig_base.hpp:72-141;
 // cota of a zero is rec(a0), an infinity with its sign)
-template <int K, bool F, class T> __device__ __forceinline__ T finish(T a0, T xr, int n)
+template <int K, bool F> __device__ __forceinline__ float finish(float a0, float xr, int n)
 {
-  using U = typename bits_of<T>::type;
-  constexpr int top = bits_of<T>::top;
+  using T = float;
+  using U = uint32_t;
+  constexpr int top = 31;
   if constexpr (K == TAN || K == TANPI || K == TAND) {
     T y = tan_eval<F>(xr);
     if (n & 1) y = -math::div(T(1), y);
@@ -610,6 +649,35 @@ template <int K, bool F, class T> __device__ __forceinline__ T finish(T a0, T xr
       return flip(v, (U)((n ^ (n >> 1)) & 1) << top);
     }
   }
+}
+
+// finish for a double: the same steps, with xr's products on the integer forms
+// when 2^-200 <= |xr| (|xr| is at most a little above pi/4), out of line otherwise.
+template <int K, bool F, class A> __device__ __forceinline__ double finish_d(double a0, double xr, int n)
+{
+  constexpr bool tk = K == TAN || K == TANPI || K == TAND, ck = K == COT || K == COTPI || K == COTD;
+  if constexpr (tk || ck) {
+    double y = tan_eval<F, A>(xr);
+    if (((n & 1) != 0) == tk) y = A::div(1.0, y);
+    if (n & 1) y = -y;
+    y = flip(y, sign_of(a0));
+    if constexpr (tk) return tan_invalid<K>(a0) ? double(NAN) : y;
+    y = cot_invalid<K>(a0) ? double(NAN) : y;
+    return f64i::is_zero(a0) ? math::div(1.0, a0) : y;
+  } else {
+    constexpr bool sk = K == SIN || K == SINPI || K == SIND;
+    const double v = sincos_eval<F, A>(((n & 1) != 0) == sk, xr);
+    return flip(v, sk ? sign_of(a0) ^ ((uint64_t)(n & 2) << 62) : (uint64_t)((n ^ (n >> 1)) & 1) << 63);
+  }
+}
+template <int K, bool F> static __device__ __noinline__ double finish_any(double a0, double xr, int n)
+{
+  return finish_d<K, F, math::f64_any>(a0, xr, n);
+}
+template <int K, bool F> __device__ __forceinline__ double finish(double a0, double xr, int n)
+{
+  if (f64i::abs_hi(xr) - 0x33700000u < 0x40000000u - 0x33700000u) return finish_d<K, F, math::f64_mid>(a0, xr, n);
+  return finish_any<K, F>(a0, xr, n);
 }
 
 // finish for two float lanes: for the sine and cosine kinds both polynomials
@@ -871,6 +939,19 @@ template <class T> __device__ __forceinline__ int reduce_low(int lv, T x, T& xr)
   const int nc = cephes(x, xc);
   xr = lv == 0 ? x : (lv == 1 ? xs : xc);
   return lv == 0 ? 0 : (lv == 1 ? 1 : nc);
+}
+// Doubles: straight is cephes with the quotient 1 and level 0 with 0, and the
+// quotient's products with the three parts of pi/2 (33 bits each) are exact, so
+// each subtraction is one fma.
+__device__ __forceinline__ int reduce_low(int lv, double x, double& xr)
+{
+  int k;
+  f64i::round_small(f64i::mul_int(x, dbits(td::twoopi)), k);    // used at level 2 only: x in (pi/2, 20 pi]
+  k = lv == 2 ? k : lv;
+  const double xi = -f64i::small_int(k);
+  const double r = __fma_rn(xi, dbits(td::pio2_2), __fma_rn(xi, dbits(td::pio2_1), x));
+  xr = __fma_rn(xi, dbits(td::pio2_3), r);
+  return k & 3;
 }
 // reduce_low for two float elements whose levels are both at most 2, on the
 // packed instructions: the straight and cephes chains are the scalar ones
