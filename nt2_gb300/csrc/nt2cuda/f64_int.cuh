@@ -33,10 +33,14 @@ namespace nt2cuda {
 namespace f64i {
 
 // --------------------------------------------------------------- words
+// (through asm: the compiler turns integer tests of a double's bits that it
+// recognises, for NaNs and zeros, back into compares on the double pipe)
 NT2_F64I uint64_t bits(double a)
 {
 #if defined(__CUDA_ARCH__)
-  return (uint64_t)__double_as_longlong(a);
+  uint64_t u;
+  asm("mov.b64 %0, %1;" : "=l"(u) : "d"(a));
+  return u;
 #else
   uint64_t u;
   memcpy(&u, &a, 8);
@@ -326,9 +330,57 @@ NT2_F64I double half(double x)
 }
 // x < c for x >= 0 or NaN without its sign, c > 0: the bits compare as integers
 NT2_F64I bool below(double x, double c) { return bits(x) < bits(c); }
+// an integer that orders doubles (not NaNs) as < does; both zeros are 0
+NT2_F64I int64_t order_key(double x)
+{
+  const int64_t m = (int64_t)(bits(x) & 0x7fffffffffffffffull);
+  return (int32_t)hi32(bits(x)) < 0 ? -m : m;
+}
 // the high word without its sign: |x| >= 2^e and non-finite tests on the top 32 bits
 NT2_F64I uint32_t abs_hi(double x) { return hi32(bits(x)) & 0x7fffffffu; }
 NT2_F64I bool is_zero(double x) { return (bits(x) << 1) == 0ull; }
+
+// --------------------------------------------------- fixed point frames
+// A block of doubles as 64-bit integers in units of 2^(F - 1075 - SH), F at
+// least every element's biased exponent: an element's significand, SH bits up,
+// shifted down by what its exponent lacks (elements more than SH bits below F
+// lose their lowest bits; zeros and far smaller ones become 0).
+NT2_F64I uint64_t shr64(uint64_t v, uint32_t n)     // 0 for n >= 64
+{
+#if defined(__CUDA_ARCH__)
+  uint64_t r;
+  asm("shr.u64 %0, %1, %2;" : "=l"(r) : "l"(v), "r"(n));
+  return r;
+#else
+  return n > 63u ? 0ull : v >> n;
+#endif
+}
+template <int SH> NT2_F64I int64_t to_fixed(double x, uint32_t F)
+{
+  const uint64_t u = bits(x);
+  const uint32_t h = hi32(u);
+  const uint64_t m = pack(lo32(u), (h & 0xfffffu) | 0x100000u) << SH;
+  const int64_t v = (int64_t)shr64(m, F - ((h >> 20) & 0x7ffu));
+  return (int32_t)h < 0 ? -v : v;
+}
+// largest biased exponent of a block; frames are made for 64 <= F < 2000 (no
+// infinities or NaNs, and the unit a normal number)
+template <int N> NT2_F64I uint32_t max_exponent(const double (&x)[N])
+{
+  uint32_t m = 0u;
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const uint32_t h = abs_hi(x[i]);
+    m = h > m ? h : m;
+  }
+  return m >> 20;
+}
+NT2_F64I bool frame_range(uint32_t F) { return F - 64u < 2000u - 64u; }
+// v * 2^n rounded to nearest; v an integer, 2^n and the product normal
+NT2_F64I double from_fixed(int64_t v, int n)
+{
+  return v ? scale((double)v, n) : 0.0;
+}
 
 }  // namespace f64i
 }  // namespace nt2cuda

@@ -129,8 +129,16 @@ template <int KIND> struct op_val {   // 0 max, 1 min, 2 prod, 3 cummax, 4 cummi
   }
   // a is the accumulator (never NaN), b the next element: NT2's max(a,b) = a > b ? a : b
   // (boost/simd/arithmetic/functions/scalar/max.hpp), except that a NaN b is skipped
+  // For doubles the comparison is of integers (magnitude, negated where the sign
+  // is set, so that the zeros are equal): two compares on the double pipe would
+  // take 32 clocks a warp, three times what the memory takes.
   template <class T> __device__ __forceinline__ static T op(T a, T b)
   {
+    if constexpr (sizeof(T) == 8 && KIND != 2) {
+      const int64_t ka = f64i::order_key(a), kb = f64i::order_key(b);
+      const bool nan = (f64i::bits(b) << 1) > 0xffe0000000000000ull;
+      return ((KIND == 0 || KIND == 3) ? ka > kb : ka < kb) || nan ? a : b;
+    }
     if constexpr (KIND == 0 || KIND == 3) return (a > b || b != b) ? a : b;
     else if constexpr (KIND == 1 || KIND == 4) return (a < b || b != b) ? a : b;
     else return math::mul(a, b);
@@ -184,17 +192,28 @@ template <bool W1, bool STDEV> struct op_moments {
     a.n = a.n + U(1);
     const U d = x - a.mean;
     if constexpr (sizeof(U) == 4) a.mean = __fmaf_rn(d, __frcp_rn(a.n), a.mean);
-    else a.mean = a.mean + d / a.n;
+    else a.mean = a.mean + math::div(d, a.n);
     a.m2 = a.m2 + d * (x - a.mean);
   }
   template <class U> __device__ __forceinline__ static state<U> merge(state<U> a, state<U> b)
   {
-    if (b.n == U(0)) return a;
-    if (a.n == U(0)) return b;
-    const U n = a.n + b.n;
-    const U d = b.mean - a.mean;
-    const U wb = b.n / n;
-    return moments<U>{n, a.mean + d * wb, a.m2 + b.m2 + d * d * a.n * wb};
+    if constexpr (sizeof(U) == 8) {
+      // five operations on the double pipe (2 a clock and SM): the counts are
+      // tested as integers, the division and products are the integer ones
+      if (f64i::is_zero(b.n)) return a;
+      if (f64i::is_zero(a.n)) return b;
+      const U n = a.n + b.n;
+      const U d = b.mean - a.mean;
+      const U wb = math::div(b.n, n);
+      return moments<U>{n, __fma_rn(d, wb, a.mean), __fma_rn(math::mul(math::mul(d, d), a.n), wb, a.m2 + b.m2)};
+    } else {
+      if (b.n == U(0)) return a;
+      if (a.n == U(0)) return b;
+      const U n = a.n + b.n;
+      const U d = b.mean - a.mean;
+      const U wb = b.n / n;
+      return moments<U>{n, a.mean + d * wb, a.m2 + b.m2 + d * d * a.n * wb};
+    }
   }
   // N values at once (N a power of two): the block's own mean and sum of
   // squared deviations in two passes over registers, then one merge, so the
@@ -234,9 +253,263 @@ template <bool W1, bool STDEV> struct op_moments {
 
 template <class Op, class T> using state_of = typename Op::template state<T>;
 
-// Operations that take a block of values at once (add_block).
-template <class Op> struct has_block_add { static constexpr bool value = false; };
-template <bool W1, bool SD> struct has_block_add<op_moments<W1, SD>> { static constexpr bool value = true; };
+// Operations that take the values of one load trip as a block, through a
+// lane-local accumulator: add(state, values) and, at the end, flush(state).
+template <class Op, class T, class E> struct block_acc { static constexpr bool value = false; };
+
+// var / stdev of floats: one Chan merge per block (op_moments::add_block).
+template <bool W1, bool SD, class E> struct block_acc<op_moments<W1, SD>, float, E> {
+  static constexpr bool value = true;
+  using S = moments<float>;
+  template <int N> __device__ __forceinline__ void add(S& a, const float (&x)[N]) { op_moments<W1, SD>::add_block(a, x); }
+  __device__ __forceinline__ void flush(S&) {}
+};
+
+// Plain sums of doubles read straight from a table: a block is summed in fixed
+// point, exactly but for what lies 2^-57 (2^-58 for 16 values) below its
+// largest element, and added with one rounding.  An addition holds GB300's
+// double pipe 16 clocks a warp, more than the 11 in which the memory delivers
+// the warp's 256 bytes; the integer form takes about 9, and three double
+// operations a block.
+template <class E> struct plain_term { static constexpr bool value = false; };
+template <class T> struct plain_term<term<T>> { static constexpr bool value = true; };
+template <class T> struct plain_term<node<tag::abs_, term<T>>> { static constexpr bool value = true; };
+template <int FIN, class E> struct block_acc<op_sum<false, FIN>, double, E> {
+  static constexpr bool value = plain_term<E>::value;
+  using S = acc<double>;
+  template <int N> __device__ __forceinline__ void add(S& a, const double (&x)[N])
+  {
+    constexpr int SH = N <= 4 ? 8 : (N <= 8 ? 7 : (N <= 16 ? 6 : 5));   // N * 2^(53+SH) <= 2^63
+    const uint32_t F = f64i::max_exponent(x);
+    if (f64i::frame_range(F)) {
+      int64_t s = 0;
+#pragma unroll
+      for (int i = 0; i < N; ++i) s += f64i::to_fixed<SH>(x[i], F);
+      a.s = math::add(a.s, f64i::from_fixed(s, (int)F - 1075 - SH));
+    } else {
+#pragma unroll
+      for (int i = 0; i < N; ++i) a.s = math::add(a.s, x[i]);
+    }
+  }
+  __device__ __forceinline__ void flush(S&) {}
+};
+
+// var / stdev of doubles: the lane keeps its values' sum and their squared
+// distances from a pivot P (the first block's mean) as exact integers in one
+// fixed point frame, two bits above the first block's largest exponent.  A
+// value costs some 28 integer instructions and no double ones (three on the
+// double pipe, 48 clocks a warp, in the blockwise two-pass form); a value
+// beyond the frame, or 512 values, closes it: its count, mean and M2 =
+// sum d^2 - (sum d)^2/n become doubles and merge into the state.  P is one of
+// n <= 512 values' block means, so (sum d)^2/n is at most about n/16 times M2
+// and the subtraction loses no more than a few bits in the worst case.
+template <bool W1, bool SD, class E> struct block_acc<op_moments<W1, SD>, double, E> {
+  static constexpr bool value = true;
+  using Op = op_moments<W1, SD>;
+  using S = moments<double>;
+  static constexpr int SH = 5;
+  int n = 0;                       // values in the frame
+  uint32_t F;                      // its exponent
+  int64_t P;                       // pivot, in the frame's units
+  int64_t s_hi;                    // sum of the values less P (128 bits)
+  uint64_t s_lo, q_hi, q_lo;       // sum of their squares (128 bits)
+
+  template <int N> __device__ __forceinline__ void add(S& a, const double (&x)[N])
+  {
+    static_assert(N <= 16 && (N & (N - 1)) == 0, "block of at most 16 values");
+    const uint32_t f = f64i::max_exponent(x);
+    if (n && (f > F || n > 512 - N)) flush(a);
+    if (f >= 2000u) {                                      // no unit for them: value by value
+#pragma unroll
+      for (int i = 0; i < N; ++i) Op::add(a, x[i]);
+      return;
+    }
+    int64_t v[N], bs = 0;
+    const bool first = n == 0;
+    if (first) F = (f > 64u ? f : 64u) + 2u;               // squares of smaller values underflow to 0 anyway
+#pragma unroll
+    for (int i = 0; i < N; ++i) {                          // below 2^58 in magnitude
+      v[i] = f64i::to_fixed<SH>(x[i], F);
+      bs += v[i];
+    }
+    if (first) {
+      P = bs / N;
+      s_hi = 0;
+      s_lo = q_hi = q_lo = 0ull;
+    }
+    bs -= P * N;
+    uint64_t c2 = 0ull, c1 = 0ull, c0 = 0ull;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      int64_t d = v[i] - P;                                // below 2^59
+      d = d < 0 ? -d : d;
+      const uint32_t lo = (uint32_t)d & 0x3fffffffu, hi = (uint32_t)(d >> 30);
+      c2 += f64i::wide(hi, hi);                            // sums of 16: below 2^62, 2^63 and 2^64
+      c1 += f64i::wide(hi, lo);
+      c0 += f64i::wide(lo, lo);
+    }
+    // (s_hi:s_lo) += bs; (q_hi:q_lo) += c2 2^60 + c1 2^31 + c0
+    const uint64_t t = s_lo + (uint64_t)bs;
+    s_hi += (bs >> 63) + (t < s_lo ? 1 : 0);
+    s_lo = t;
+    add_q(c2 >> 4, c2 << 60);
+    add_q(c1 >> 33, c1 << 31);
+    add_q(0ull, c0);
+    n += N;
+  }
+  __device__ __forceinline__ void add_q(uint64_t hi, uint64_t lo)
+  {
+    const uint64_t t = q_lo + lo;
+    q_hi += hi + (t < lo ? 1ull : 0ull);
+    q_lo = t;
+  }
+  __device__ __forceinline__ static double to_double(uint64_t hi, uint64_t lo)
+  {
+    return __fma_rn((double)hi, 18446744073709551616.0, (double)lo);
+  }
+  __device__ __forceinline__ void flush(S& a)
+  {
+    if (n) a = closed(a, n, F, P, s_hi, s_lo, q_hi, q_lo);
+    n = 0;
+  }
+  static __device__ __noinline__ S closed(S a, int n, uint32_t F, int64_t P, int64_t s_hi, uint64_t s_lo, uint64_t q_hi,
+                                          uint64_t q_lo)
+  {
+    const double cnt = (double)n;
+    const bool neg = s_hi < 0;
+    const uint64_t lo = neg ? 0ull - s_lo : s_lo;
+    const uint64_t hi = neg ? ~(uint64_t)s_hi + (s_lo == 0ull ? 1ull : 0ull) : (uint64_t)s_hi;
+    const double sd = neg ? -to_double(hi, lo) : to_double(hi, lo);        // sum of (value - P)
+    const double md = math::div(sd, cnt);
+    const double m2 = fmax(__fma_rn(-sd, md, to_double(q_hi, q_lo)), 0.0);
+    const double unit = f64i::from_bits((uint64_t)(F - 1075u - (uint32_t)SH + 1023u) << 52);
+    return Op::merge(a, S{cnt, ((double)P + md) * unit, m2 * unit * unit});
+  }
+};
+
+// The same for a whole warp folding one segment (k_inner): the frame, its pivot
+// and its closing are the warp's, the lanes' sums meet as integers, and a trip
+// may be ragged (values a lane does not have add nothing), so no value and no
+// lane costs a double operation of its own.
+template <class Op, int N> struct warp_frame {
+  using S = moments<double>;
+  static constexpr int SH = 5, LOG = N == 16 ? 4 : (N == 8 ? 3 : (N == 4 ? 2 : -1));
+  static_assert(LOG > 0, "4, 8 or 16 values a lane");
+  int n = 0;                       // values of this lane in the frame
+  bool open = false;               // the warp has one
+  uint32_t F;
+  int64_t P, s_hi;
+  uint64_t s_lo, q_hi, q_lo;
+  S lone = S{0.0, 0.0, 0.0};       // values no frame takes (infinities, NaNs, the largest): this lane's
+  bool any_lone = false;
+
+  // cnt <= N values of this lane, a prefix of x; called by the whole warp
+  __device__ __forceinline__ void add(S& a, const double (&x)[N], int cnt)
+  {
+    uint32_t f = 0u;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const uint32_t h = f64i::abs_hi(x[i]);
+      if (i < cnt && h > f) f = h;
+    }
+    f = __reduce_max_sync(0xffffffffu, f >> 20);
+    if (open && (f > F || __any_sync(0xffffffffu, n > 512 - N))) close(a);
+    if (f >= 2000u) {
+#pragma unroll 1
+      for (int i = 0; i < cnt; ++i) Op::add(lone, x[i]);
+      any_lone = true;
+      return;
+    }
+    const bool first = !open;
+    if (first) F = (f > 64u ? f : 64u) + 2u;               // squares of smaller values underflow to 0 anyway
+    int64_t v[N], bs = 0;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {                          // below 2^58 in magnitude
+      v[i] = i < cnt ? f64i::to_fixed<SH>(x[i], F) : 0;
+      bs += v[i];
+    }
+    if (first) {                                           // the pivot: the trip's mean (roughly, if it is ragged)
+      const int total = (int)__reduce_add_sync(0xffffffffu, (unsigned)cnt);
+      P = bs >> (5 + LOG);
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) P += __shfl_xor_sync(0xffffffffu, P, off);
+      if (total < 32 * N) P = (int64_t)((float)P * ((float)(32 * N) / (float)total));
+      s_hi = 0;
+      s_lo = q_hi = q_lo = 0ull;
+      n = 0;
+      open = true;
+    }
+    bs -= P * cnt;
+    uint64_t c2 = 0ull, c1 = 0ull, c0 = 0ull;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      int64_t d = i < cnt ? v[i] - P : 0;                  // below 2^59
+      d = d < 0 ? -d : d;
+      const uint32_t lo = (uint32_t)d & 0x3fffffffu, hi = (uint32_t)(d >> 30);
+      c2 += f64i::wide(hi, hi);                            // sums of 16: below 2^62, 2^63 and 2^64
+      c1 += f64i::wide(hi, lo);
+      c0 += f64i::wide(lo, lo);
+    }
+    const uint64_t t = s_lo + (uint64_t)bs;
+    s_hi += (bs >> 63) + (t < s_lo ? 1 : 0);
+    s_lo = t;
+    add_q(c2 >> 4, c2 << 60);
+    add_q(c1 >> 33, c1 << 31);
+    add_q(0ull, c0);
+    n += cnt;
+  }
+  __device__ __forceinline__ void add_q(uint64_t hi, uint64_t lo)
+  {
+    const uint64_t t = q_lo + lo;
+    q_hi += hi + (t < lo ? 1ull : 0ull);
+    q_lo = t;
+  }
+  // Sum the lanes' integers (the squares in 160 bits) and merge; every lane gets the result.
+  __device__ __forceinline__ void close(S& a)
+  {
+    a = closed(a, n, F, P, s_hi, s_lo, q_hi, q_lo);
+    open = false;
+    n = 0;
+  }
+  static __device__ __noinline__ S closed(S a, int n, uint32_t F, int64_t P, int64_t s_hi, uint64_t s_lo, uint64_t q_hi,
+                                          uint64_t q_lo)
+  {
+    uint32_t q_x = 0u;
+#pragma unroll 1
+    for (int off = 16; off > 0; off >>= 1) {
+      const uint64_t sl = __shfl_xor_sync(0xffffffffu, s_lo, off), ql = __shfl_xor_sync(0xffffffffu, q_lo, off);
+      const int64_t sh = __shfl_xor_sync(0xffffffffu, s_hi, off);
+      const uint64_t qh = __shfl_xor_sync(0xffffffffu, q_hi, off);
+      const uint32_t qx = __shfl_xor_sync(0xffffffffu, q_x, off);
+      n += __shfl_xor_sync(0xffffffffu, n, off);
+      s_lo += sl;
+      s_hi += sh + (s_lo < sl ? 1 : 0);
+      q_lo += ql;
+      const uint64_t c = q_lo < ql ? 1ull : 0ull, h1 = q_hi + qh, h2 = h1 + c;
+      q_x += qx + (h1 < qh ? 1u : 0u) + (h2 < c ? 1u : 0u);
+      q_hi = h2;
+    }
+    const double two64 = 18446744073709551616.0, cnt = (double)n;
+    const bool neg = s_hi < 0;
+    const uint64_t lo = neg ? 0ull - s_lo : s_lo;
+    const uint64_t hi = neg ? ~(uint64_t)s_hi + (s_lo == 0ull ? 1ull : 0ull) : (uint64_t)s_hi;
+    const double mag = __fma_rn((double)hi, two64, (double)lo), sd = neg ? -mag : mag;    // sum of (value - P)
+    const double q = __fma_rn(__fma_rn((double)q_x, two64, (double)q_hi), two64, (double)q_lo);
+    const double md = math::div(sd, cnt);
+    const double m2 = fmax(__fma_rn(-sd, md, q), 0.0);
+    const double unit = f64i::from_bits((uint64_t)(F - 1075u - (uint32_t)SH + 1023u) << 52);
+    return Op::merge(a, S{cnt, ((double)P + md) * unit, m2 * unit * unit});
+  }
+};
+template <class Op, class T> struct warp_framed { static constexpr bool value = false; };
+template <bool W1, bool SD> struct warp_framed<op_moments<W1, SD>, double> { static constexpr bool value = true; };
+
+// Resident blocks asked for: four (64 registers; six for short columns, which
+// take few loads and wait for them), two where a lane keeps the
+// integer frame of var/stdev beside its 16 values.
+template <class Op, class T, int U> struct fold_min_blocks { static constexpr int value = U <= 4 ? 6 : 4; };
+template <bool W1, bool SD, int U> struct fold_min_blocks<op_moments<W1, SD>, double, U> { static constexpr int value = U <= 4 ? 3 : 2; };
+
 template <class Op, class T> using out_of = typename Op::template out_t<T>;
 
 // Butterfly over the warp; every lane ends with the same value.
@@ -249,6 +522,27 @@ template <class Op, class T> __device__ __forceinline__ state_of<Op, T> warp_mer
     a = ((threadIdx.x & 31) & off) ? Op::merge(o, a) : Op::merge(a, o);
   }
   return a;
+}
+
+// Merge n partials p[0], p[stride], ... in index order, with 8 loads in
+// flight at a time (the merge is at the tail of the kernel, where serial L2
+// round trips would show).
+template <class Op, class T, int N = 8>
+__device__ __forceinline__ state_of<Op, T> merge_partials(const state_of<Op, T>* p, size_t n, size_t stride)
+{
+  state_of<Op, T> m = Op::template init<T>();
+  size_t q = 0;
+#pragma unroll 1
+  for (; q + N <= n; q += N) {
+    state_of<Op, T> v[N];
+#pragma unroll
+    for (int k = 0; k < N; ++k) v[k] = Op::ldcg(p + (q + k) * stride);
+#pragma unroll
+    for (int k = 0; k < N; ++k) m = Op::merge(m, v[k]);
+  }
+#pragma unroll 1
+  for (; q < n; ++q) m = Op::merge(m, Op::ldcg(p + q * stride));
+  return m;
 }
 
 // Folds of zero elements: every output is finish(neutral).
@@ -269,8 +563,12 @@ struct inner_shape {
   size_t rows, cols, seg, splits;
 };
 
+// fold_min_blocks: left to itself the
+// compiler keeps 48 registers, 32 where a lane loads single elements, and
+// issues the U loads a few at a time (sum(A,1) of 8192 x 4096 floats 24.5 us,
+// now 21.5; 300001 x 50, single elements, 27.8 us, now 14.8).
 template <class Op, int V, int U, class T, class E>
-__global__ void __launch_bounds__(256) k_inner(E e, inner_shape sh, out_of<Op, T>* __restrict__ out,
+__global__ void __launch_bounds__(256, (fold_min_blocks<Op, T, U>::value)) k_inner(E e, inner_shape sh, out_of<Op, T>* __restrict__ out,
                                                state_of<Op, T>* __restrict__ partials, unsigned* __restrict__ counters)
 {
   const int lane = threadIdx.x & 31;
@@ -282,7 +580,7 @@ __global__ void __launch_bounds__(256) k_inner(E e, inner_shape sh, out_of<Op, T
     const size_t w = (size_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     constexpr int LANES_PER_LINE = (V * (int)sizeof(T)) >= 128 ? 1 : 128 / (V * (int)sizeof(T));
     if (w < units && V > 1 && lane % LANES_PER_LINE == 0) {
-      const size_t j = w / sh.splits, r0 = (w % sh.splits) * sh.seg;
+      const size_t j = sh.splits == 1 ? w : w / sh.splits, r0 = (w - j * sh.splits) * sh.seg;
       const size_t r1 = (r0 + sh.seg < sh.rows) ? r0 + sh.seg : sh.rows;
       const size_t g1 = r1 / V;
 #pragma unroll
@@ -294,27 +592,65 @@ __global__ void __launch_bounds__(256) k_inner(E e, inner_shape sh, out_of<Op, T
   }
   nt2cuda::mem::pdl_begin();
   for (size_t w = (size_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < units; w += warps_total) {
-    const size_t j = w / sh.splits, sp = w % sh.splits;
+    const size_t j = sh.splits == 1 ? w : w / sh.splits, sp = w - j * sh.splits;   // a 64-bit division is long
     const size_t r0 = sp * sh.seg;
     const size_t r1 = (r0 + sh.seg < sh.rows) ? r0 + sh.seg : sh.rows;
     const size_t base = j * sh.rows;
+    constexpr bool BLK = block_acc<Op, T, E>::value;
+    block_acc<Op, T, E> ba;
     state_of<Op, T> a[V];
 #pragma unroll
     for (int l = 0; l < V; ++l) a[l] = Op::template init<T>();
-    // full V-groups
     const size_t g0 = r0 / V, g1 = r1 / V;   // r0 is a multiple of V
-    size_t g = g0 + lane;
+    if constexpr (warp_framed<Op, T>::value) {
+      constexpr int N = U * V;
+      warp_frame<Op, N> wf;
+      state_of<Op, T> t = Op::template init<T>();
+      // the V-groups, and (r1 % V != 0 only at a column's end) the ragged rest, one value per lane
+      for (size_t g = g0; g < g1; g += (size_t)U * 32) {
+        T x[N];
+        int have = 0;
+        regs<E, V> rr[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const bool in = g + (size_t)u * 32 + lane < g1;
+          have += in ? V : 0;
+          if (in) rr[u].template load<true>(e, base + (g + (size_t)u * 32 + lane) * V);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+          for (int l = 0; l < V; ++l) x[u * V + l] = u * V + l < have ? (T)rr[u].template get<false>(e, l) : T(0);
+        wf.add(t, x, have);
+      }
+      for (size_t r = g1 * V; r < r1; r += 32) {
+        T x[N] = {};
+        const int have = r + lane < r1 ? 1 : 0;
+        if (have) {
+          regs<E, 1> rr;
+          rr.template load<false>(e, base + r + lane);
+          x[0] = (T)rr.template get<false>(e, 0);
+        }
+        wf.add(t, x, have);
+      }
+      if (wf.open) wf.close(t);
+      if (wf.any_lone) t = Op::merge(t, warp_merge<Op, T>(wf.lone));
+      a[0] = t;
+    }
+    // full V-groups
+    size_t g = warp_framed<Op, T>::value ? g1 : g0 + lane;
+    if constexpr (!warp_framed<Op, T>::value) {
     for (; g + (size_t)(U - 1) * 32 < g1; g += (size_t)U * 32) {
       regs<E, V> rr[U];
 #pragma unroll
       for (int u = 0; u < U; ++u) rr[u].template load<true>(e, base + (g + (size_t)u * 32) * V);
-      if constexpr (has_block_add<Op>::value && ((U * V) & (U * V - 1)) == 0) {
+      if constexpr (BLK) {
         T blk[U * V];
 #pragma unroll
         for (int u = 0; u < U; ++u)
 #pragma unroll
           for (int l = 0; l < V; ++l) blk[u * V + l] = (T)rr[u].template get<false>(e, l);
-        Op::add_block(a[0], blk);
+        ba.add(a[0], blk);
       } else {
 #pragma unroll
         for (int u = 0; u < U; ++u)
@@ -322,22 +658,62 @@ __global__ void __launch_bounds__(256) k_inner(E e, inner_shape sh, out_of<Op, T
           for (int l = 0; l < V; ++l) Op::add(a[l], (T)rr[u].template get<false>(e, l));
       }
     }
-    for (; g < g1; g += 32) {
-      regs<E, V> rr;
-      rr.template load<true>(e, base + g * V);
+    // what is left of the segment: four groups at a time, then at most three
+    if constexpr (U > 4) {
+#pragma unroll 1
+      for (; g + (size_t)3 * 32 < g1; g += (size_t)4 * 32) {
+        regs<E, V> rr[4];
 #pragma unroll
-      for (int l = 0; l < V; ++l) Op::add(a[l], (T)rr.template get<false>(e, l));
+        for (int u = 0; u < 4; ++u) rr[u].template load<true>(e, base + (g + (size_t)u * 32) * V);
+        if constexpr (BLK) {
+          T blk[4 * V];
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int l = 0; l < V; ++l) blk[u * V + l] = (T)rr[u].template get<false>(e, l);
+          ba.add(a[0], blk);
+        } else {
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int l = 0; l < V; ++l) Op::add(a[l], (T)rr[u].template get<false>(e, l));
+        }
+      }
+    }
+    {
+      regs<E, V> rr[3];
+#pragma unroll
+      for (int u = 0; u < 3; ++u)
+        if (g + (size_t)u * 32 < g1) rr[u].template load<true>(e, base + (g + (size_t)u * 32) * V);
+      // a loop over the trips the warp has, the loaded values moving up: unrolled,
+      // each add becomes a predicated one, and those that are off still take
+      // their turn on the double pipe
+      const size_t gw = g - lane;
+#pragma unroll 1
+      for (size_t q = gw; q < g1; q += 32) {
+        if (q + lane < g1) {
+#pragma unroll
+          for (int l = 0; l < V; ++l) Op::add(a[l], (T)rr[0].template get<false>(e, l));
+        }
+        rr[0] = rr[1];
+        rr[1] = rr[2];
+      }
+    }
+    if constexpr (BLK) ba.flush(a[0]);
     }
     // ragged end of the segment (only when rows % V != 0 or V == 1)
-    for (size_t r = g1 * V + lane; r < r1; r += 32) {
-      regs<E, 1> rr;
-      rr.template load<false>(e, base + r);
-      Op::add(a[0], (T)rr.template get<false>(e, 0));
-    }
+    if constexpr (!warp_framed<Op, T>::value)
+      for (size_t r = g1 * V + lane; r < r1; r += 32) {
+        regs<E, 1> rr;
+        rr.template load<false>(e, base + r);
+        Op::add(a[0], (T)rr.template get<false>(e, 0));
+      }
     state_of<Op, T> t = a[0];
+    if constexpr (!warp_framed<Op, T>::value) {
 #pragma unroll
-    for (int l = 1; l < V; ++l) t = Op::merge(t, a[l]);
-    t = warp_merge<Op, T>(t);
+      for (int l = 1; l < V; ++l) t = Op::merge(t, a[l]);
+      t = warp_merge<Op, T>(t);
+    }
     if (sh.splits == 1) {
       if (lane == 0) out[j] = Op::finish(t, sh.rows);
       continue;
@@ -353,10 +729,10 @@ __global__ void __launch_bounds__(256) k_inner(E e, inner_shape sh, out_of<Op, T
     last = __shfl_sync(0xffffffffu, last, 0);
     if (!last) continue;
     __threadfence();
-    // combine the column's partials in segment order: lane k folds
-    // segments k, k+32, ... then the butterfly merges lanes in order
-    state_of<Op, T> c = Op::template init<T>();
-    for (size_t q = lane; q < sh.splits; q += 32) c = Op::merge(c, Op::ldcg(partials + j * sh.splits + q));
+    // combine the column's partials in a fixed order: lane k folds segments
+    // k, k+32, ..., then the butterfly merges lanes in order
+    const size_t mine = sh.splits > (size_t)lane ? (sh.splits - lane + 31) / 32 : 0;
+    state_of<Op, T> c = merge_partials<Op, T>(partials + j * sh.splits + lane, mine, 32);
     c = warp_merge<Op, T>(c);
     if (lane == 0) out[j] = Op::finish(c, sh.rows);
   }
@@ -389,8 +765,11 @@ struct outer_shape {
   size_t rows, cols, cchunk, splits, strips;
 };
 
+// fold_min_blocks: left to itself the compiler keeps 48 registers
+// (32 where a lane loads single elements) and issues the U loads a few at a time
+// (8192 x 4096 floats 24.2 us, now 22.5; 10001 x 777 floats 20.3, now 9.7).
 template <class Op, int V, int U, class T, class E>
-__global__ void __launch_bounds__(256) k_outer(E e, outer_shape sh, out_of<Op, T>* __restrict__ out,
+__global__ void __launch_bounds__(256, (fold_min_blocks<Op, T, U>::value)) k_outer(E e, outer_shape sh, out_of<Op, T>* __restrict__ out,
                                                state_of<Op, T>* __restrict__ partials, unsigned* __restrict__ counters)
 {
   using S = state_of<Op, T>;
@@ -424,6 +803,8 @@ __global__ void __launch_bounds__(256) k_outer(E e, outer_shape sh, out_of<Op, T
     const size_t m0 = sp * sh.cchunk;
     const size_t m1 = (m0 + sh.cchunk < sh.cols) ? m0 + sh.cchunk : sh.cols;
     const bool full = row0 + V <= sh.rows;
+    constexpr bool BLK = block_acc<Op, T, E>::value;
+    block_acc<Op, T, E> ba[V];
     S a[V];
 #pragma unroll
     for (int l = 0; l < V; ++l) a[l] = Op::template init<T>();
@@ -433,14 +814,14 @@ __global__ void __launch_bounds__(256) k_outer(E e, outer_shape sh, out_of<Op, T
         regs<E, V> rr[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) rr[u].template load<true>(e, (m + (size_t)u * 8) * sh.rows + row0);
-        if constexpr (has_block_add<Op>::value && (U & (U - 1)) == 0) {
+        if constexpr (BLK) {
           // lane slot l is one row: its U values of this trip form a block
 #pragma unroll
           for (int l = 0; l < V; ++l) {
             T blk[U];
 #pragma unroll
             for (int u = 0; u < U; ++u) blk[u] = (T)rr[u].template get<false>(e, l);
-            Op::add_block(a[l], blk);
+            ba[l].add(a[l], blk);
           }
         } else {
 #pragma unroll
@@ -449,12 +830,44 @@ __global__ void __launch_bounds__(256) k_outer(E e, outer_shape sh, out_of<Op, T
             for (int l = 0; l < V; ++l) Op::add(a[l], (T)rr[u].template get<false>(e, l));
         }
       }
-      for (; m < m1; m += 8) {
-        regs<E, V> rr;
-        rr.template load<true>(e, m * sh.rows + row0);
+      if constexpr (U > 4) {
+#pragma unroll 1
+        for (; m + (size_t)3 * 8 < m1; m += (size_t)4 * 8) {
+          regs<E, V> rr[4];
 #pragma unroll
-        for (int l = 0; l < V; ++l) Op::add(a[l], (T)rr.template get<false>(e, l));
+          for (int u = 0; u < 4; ++u) rr[u].template load<true>(e, (m + (size_t)u * 8) * sh.rows + row0);
+          if constexpr (BLK) {
+#pragma unroll
+            for (int l = 0; l < V; ++l) {
+              T blk[4];
+#pragma unroll
+              for (int u = 0; u < 4; ++u) blk[u] = (T)rr[u].template get<false>(e, l);
+              ba[l].add(a[l], blk);
+            }
+          } else {
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+#pragma unroll
+              for (int l = 0; l < V; ++l) Op::add(a[l], (T)rr[u].template get<false>(e, l));
+          }
+        }
       }
+      {
+        regs<E, V> rr[3];
+#pragma unroll
+        for (int u = 0; u < 3; ++u)
+          if (m + (size_t)u * 8 < m1) rr[u].template load<true>(e, (m + (size_t)u * 8) * sh.rows + row0);
+#pragma unroll 1
+        for (size_t q = m; q < m1; q += 8) {      // a loop, not predicated adds: see k_inner
+#pragma unroll
+          for (int l = 0; l < V; ++l) Op::add(a[l], (T)rr[0].template get<false>(e, l));
+          rr[0] = rr[1];
+          rr[1] = rr[2];
+        }
+      }
+      if constexpr (BLK)
+#pragma unroll
+        for (int l = 0; l < V; ++l) ba[l].flush(a[l]);
     } else if (row0 < sh.rows) {
       for (size_t m = m0 + warp; m < m1; m += 8)
 #pragma unroll
@@ -492,17 +905,17 @@ __global__ void __launch_bounds__(256) k_outer(E e, outer_shape sh, out_of<Op, T
     __syncthreads();
     if (is_last) {
       __threadfence();
+      // merge the strip's chunks in a fixed order: the threads are 256/STRIP groups
+      // over the rows, group g takes chunks g, g + G, ..., then the groups in order
+      constexpr int G = 256 / STRIP;
+      const int r = threadIdx.x % STRIP, g = threadIdx.x / STRIP;
+      const size_t mine = sh.splits > (size_t)g ? (sh.splits - g + G - 1) / G : 0;
+      red[g][r] = merge_partials<Op, T, 4>(partials + (strip * sh.splits + g) * STRIP + r, mine, (size_t)G * STRIP);
+      __syncthreads();
       if (threadIdx.x < STRIP && row < sh.rows) {
-        S c = Op::template init<T>();
-        size_t q = 0;
-        for (; q + 8 <= sh.splits; q += 8) {
-          S v[8];
+        S c = red[0][threadIdx.x];
 #pragma unroll
-          for (int k = 0; k < 8; ++k) v[k] = Op::ldcg(partials + (strip * sh.splits + q + k) * STRIP + threadIdx.x);
-#pragma unroll
-          for (int k = 0; k < 8; ++k) c = Op::merge(c, v[k]);
-        }
-        for (; q < sh.splits; ++q) c = Op::merge(c, Op::ldcg(partials + (strip * sh.splits + q) * STRIP + threadIdx.x));
+        for (int w = 1; w < G; ++w) c = Op::merge(c, red[w][threadIdx.x]);
         out[row] = Op::finish(c, sh.cols);
       }
     }

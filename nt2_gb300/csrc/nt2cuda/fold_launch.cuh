@@ -29,8 +29,25 @@ template <class E> bool expr_aligned(const E& e)
   return ok;
 }
 
-// Segment length of one warp's share of a column: 128 vector groups per lane.
-template <class T> constexpr size_t inner_seg() { return (size_t)32 * (16 / sizeof(T)) * 128; }
+// How inner_fold cuts columns into segments, one to a warp: into about
+// `kInnerUnits` segments in all, 24 a SM with 16-byte loads and 16 with single
+// elements, so that a few long columns fill the chip too (3333333 x 1 floats:
+// 44 us with segments of 16384, 10.5 with 2432 of them), but never below eight
+// loads a lane, and at most kInnerSplits to a column, as one warp merges them.
+// The cut depends on the table's shape alone: results are reproducible.
+// (var/stdev of doubles: 1216, 8 a SM, as merging their partials takes longer.)
+constexpr size_t kInnerUnits = 3648, kInnerUnitsScalar = 2432, kInnerUnitsFramed = 1216, kInnerSplits = 2432;
+constexpr size_t kInnerWhole = 4096;     // 16-byte groups of the longest column folded whole under capture
+template <class Op, class T> inline size_t inner_seg(size_t rows, size_t cols, bool vec)
+{
+  const size_t lanes = vec ? 32 * (16 / sizeof(T)) : 32;
+  const size_t units = warp_framed<Op, T>::value ? kInnerUnitsFramed : (vec ? kInnerUnits : kInnerUnitsScalar);
+  size_t splits = (units + cols / 2) / cols;              // rounded: half a segment more or less a column
+  if (splits < 1) splits = 1;
+  if (splits > kInnerSplits) splits = kInnerSplits;
+  size_t seg = round_up((rows + splits - 1) / splits, lanes);
+  return seg < lanes * 8 ? lanes * 8 : seg;
+}
 
 // Which kernels serve the folds of a table or of a product of two tables:
 //   0 (auto): TMA-staged for long columns (inner_fold, rows >= 2^16), the
@@ -59,15 +76,18 @@ template <class T> inline const T* first_term(const node<tag::multiplies_, term<
 template <class T> inline const T* second_term(const term<T>&) { return nullptr; }
 template <class T> inline const T* second_term(const node<tag::multiplies_, term<T>, term<T>>& n) { return n.b.p; }
 
-// Loads in flight per lane in the register-pipelined kernels: 16 (8 left the
-// 134 MB folds at 71% of the copy peak, 16 reaches 75-77%, 32 adds nothing),
-// or 8 for var/stdev, whose block updates (add_block) hold the loaded values
-// until the block's mean is known.
-template <class Op> struct fold_unroll { static constexpr int value = 16; };
-template <bool W1, bool SD> struct fold_unroll<op_moments<W1, SD>> { static constexpr int value = 8; };
-// outer_fold keeps V rows' states per lane: var/stdev there take 4 columns a trip
-template <class Op> struct outer_unroll { static constexpr int value = fold_unroll<Op>::value; };
-template <bool W1, bool SD> struct outer_unroll<op_moments<W1, SD>> { static constexpr int value = 4; };
+// Loads in flight per lane in the register-pipelined kernels: 16, or 8 where a
+// trip's values form a block (block_acc): its values stay in registers.
+template <class Op, class T, class E> struct fold_unroll {
+  static constexpr int value = block_acc<Op, T, E>::value ? 8 : 16;
+};
+// outer_fold keeps V rows' states per lane: var/stdev of floats there take 4 columns a trip
+template <class Op, class T, class E> struct outer_unroll { static constexpr int value = fold_unroll<Op, T, E>::value; };
+template <bool W1, bool SD, class E> struct outer_unroll<op_moments<W1, SD>, float, E> { static constexpr int value = 4; };
+// Tables whose rows or alignment rule out 16-byte loads: one element per lane
+// and load, so as many loads in flight again.
+constexpr int kScalarUnroll = 16;
+constexpr size_t kOuterUnits = 608;
 
 template <class Op, class T> cudaError_t fold_empty(out_of<Op, T>* out, size_t count, cudaStream_t s)
 {
@@ -85,7 +105,10 @@ cudaError_t inner_fold(const E& e, size_t rows, size_t cols, out_of<Op, T>* out,
     // auto: long columns only; a short column's tiles are too few to amortise the block barriers
     const int path = fold_path().load(std::memory_order_relaxed);
     const size_t min_rows = path == 2 ? 32 : ((size_t)1 << 16);
-    if (path != 1 && rows >= min_rows && cols > 0 && out && rows % VV == 0 && expr_aligned(e) &&
+    // (var/stdev of doubles: the register-pipelined kernel, whose integer frames
+    // leave the staged one a single block per SM)
+    constexpr bool staged = !(std::is_same<S, moments<double>>::value);
+    if (path != 1 && (staged || path == 2) && rows >= min_rows && cols > 0 && out && rows % VV == 0 && expr_aligned(e) &&
         std::is_same<typename value_of<E>::type, T>::value)
       return inner_fold_tma<Op, T>(first_term(e), second_term(e), rows, cols, out, s);
   }
@@ -104,8 +127,13 @@ cudaError_t inner_fold(const E& e, size_t rows, size_t cols, out_of<Op, T>* out,
   inner_shape sh;
   sh.rows = rows;
   sh.cols = cols;
-  sh.seg = inner_seg<T>();
+  sh.seg = inner_seg<Op, T>(rows, cols, vec);
   sh.splits = (rows + sh.seg - 1) / sh.seg;
+  // a stream captured before its scratch was allocated: columns of one warp each
+  if (sh.splits > 1 && rows <= kInnerWhole * VV && fold_scratch_barred(s, cols, cols * sh.splits, sizeof(S))) {
+    sh.seg = round_up(rows, 32 * VV);
+    sh.splits = 1;
+  }
   S* partials = nullptr;
   unsigned* counters = nullptr;
   if (sh.splits > 1) {
@@ -118,9 +146,14 @@ cudaError_t inner_fold(const E& e, size_t rows, size_t cols, out_of<Op, T>* out,
   E ec = e;
   out_of<Op, T>* o = out;
   void* args[] = {&ec, &sh, &o, &partials, &counters};
-  // launch_persistent counts threads; a unit is one warp
-  if (vec) return (launch_persistent(k_inner<Op, VV, fold_unroll<Op>::value, T, E>, units * 32, 128, 4, s, args));
-  return (launch_persistent(k_inner<Op, 1, 4, T, E>, units * 32, 256, 4, s, args));
+  // launch_persistent counts threads; a unit is one warp.  Columns of at most
+  // eight loads a lane take the kernel with four in flight.
+  if (rows <= (size_t)32 * (vec ? VV : 1) * 8) {
+    if (vec) return (launch_persistent(k_inner<Op, VV, 4, T, E>, units * 32, 128, 4, s, args));
+    return (launch_persistent(k_inner<Op, 1, 4, T, E>, units * 32, 128, 4, s, args));
+  }
+  if (vec) return (launch_persistent(k_inner<Op, VV, fold_unroll<Op, T, E>::value, T, E>, units * 32, 128, 4, s, args));
+  return (launch_persistent(k_inner<Op, 1, kScalarUnroll, T, E>, units * 32, 128, 4, s, args));
 }
 
 template <class Op, class T, class E>
@@ -146,12 +179,12 @@ cudaError_t outer_fold(const E& e, size_t rows, size_t cols, out_of<Op, T>* out,
   sh.rows = rows;
   sh.cols = cols;
   sh.strips = (rows + STRIP - 1) / STRIP;
-  // about 512 blocks in all, so the grid fits in one wave of resident blocks
-  // (the split depends only on the shape, so results stay reproducible)
+  // as many chunks as keep the blocks within 608, four a SM: one wave, every
+  // block at once (8192 x 4096 floats in 640 blocks takes 29.8 us); the split
+  // depends only on the shape, so results stay reproducible
   {
-    const size_t want_splits = (512 + sh.strips - 1) / sh.strips;
-    size_t cchunk = (cols + want_splits - 1) / want_splits;
-    cchunk = (cchunk + 63) / 64 * 64;
+    const size_t want = sh.strips < kOuterUnits ? kOuterUnits / sh.strips : 1;
+    const size_t cchunk = round_up((cols + want - 1) / want, 8);
     sh.cchunk = cchunk < 64 ? 64 : cchunk;
   }
   sh.splits = (cols + sh.cchunk - 1) / sh.cchunk;
@@ -167,8 +200,8 @@ cudaError_t outer_fold(const E& e, size_t rows, size_t cols, out_of<Op, T>* out,
   E ec = e;
   out_of<Op, T>* o = out;
   void* args[] = {&ec, &sh, &o, &partials, &counters};
-  if (vec) return (launch_persistent(k_outer<Op, VV, outer_unroll<Op>::value, T, E>, units * 256, 256, 4, s, args));
-  return (launch_persistent(k_outer<Op, 1, 4, T, E>, units * 256, 256, 4, s, args));
+  if (vec) return (launch_persistent(k_outer<Op, VV, outer_unroll<Op, T, E>::value, T, E>, units * 256, 256, 4, s, args));
+  return (launch_persistent(k_outer<Op, 1, kScalarUnroll, T, E>, units * 256, 256, 4, s, args));
 }
 
 }  // namespace fold

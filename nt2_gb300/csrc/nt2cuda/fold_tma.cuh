@@ -63,25 +63,6 @@ template <class T> __device__ __forceinline__ T quiet_nan()
   else return __longlong_as_double(0x7ff8000000000000ll);
 }
 
-// Merge n partials p[0], p[stride], ... in index order, with 8 loads in
-// flight at a time (the merge is at the tail of the kernel, where serial L2
-// round trips would show).
-template <class Op, class T>
-__device__ __forceinline__ state_of<Op, T> merge_partials(const state_of<Op, T>* p, size_t n, size_t stride)
-{
-  state_of<Op, T> m = Op::template init<T>();
-  size_t q = 0;
-  for (; q + 8 <= n; q += 8) {
-    state_of<Op, T> v[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) v[k] = Op::ldcg(p + (q + k) * stride);
-#pragma unroll
-    for (int k = 0; k < 8; ++k) m = Op::merge(m, v[k]);
-  }
-  for (; q < n; ++q) m = Op::merge(m, Op::ldcg(p + q * stride));
-  return m;
-}
-
 // Merge v[threadIdx.x] over the block in a fixed order; thread 0 gets the result.
 template <class Op, class T>
 __device__ __forceinline__ state_of<Op, T> block_merge(state_of<Op, T> v, state_of<Op, T>* red)
@@ -105,6 +86,29 @@ struct inner_tma_shape {
   size_t fail_unit;
   uint32_t wait_rounds;
 };
+
+// Elements of a unit.  The blocks are resident all at once (2 a SM of 152 with
+// two tables, 3 with one) and stream one tile after another, so the longest
+// block's elements decide: the columns are cut into the number of segments, of
+// the candidates that give every block 1, 2, ... 8 of them, with the fewest
+// elements to a block, half a tile counted for each unit's start and end.
+// (dot over 2^26 floats: 91.5 us in 1024 units of 16 tiles, 80.0 in 304;
+// 4000000 floats: 17.7 us in 62 units, 7.8 in 456.)  At least a quarter tile.
+template <class T> inline size_t inner_tma_seg(size_t rows, size_t cols, int tables)
+{
+  constexpr size_t TILE = kTmaTileBytes / sizeof(T), VV = 16 / sizeof(T);
+  const size_t slots = tables == 2 ? 304 : 456;
+  size_t best = rows, best_cost = ~(size_t)0;
+  for (size_t k = 1; k <= 8; ++k) {
+    const size_t per_col = k * slots / cols > 1 ? k * slots / cols : 1;
+    size_t seg = ((rows + per_col - 1) / per_col + VV - 1) / VV * VV;
+    if (seg < TILE / 4) seg = TILE / 4;
+    const size_t units = cols * ((rows + seg - 1) / seg);
+    const size_t cost = (units + slots - 1) / slots * (seg + TILE / 2);
+    if (cost < best_cost) { best = seg; best_cost = cost; }
+  }
+  return best;
+}
 
 // A block that gave up: count it, then let every unit it still owns arrive
 // poisoned (a column folded in one piece gets NaN at once; a split column's
@@ -131,12 +135,20 @@ __device__ void inner_give_up(const inner_tma_shape& sh, size_t cu, O* out, unsi
 
 template <class T> __host__ __device__ constexpr int inner_tile() { return kTmaTileBytes / (int)sizeof(T); }
 
-template <class T>
-__device__ __forceinline__ size_t inner_unit_tiles(const inner_tma_shape& sh, size_t u)
+// A unit's column, its elements' offset from the table's start, their count and
+// its tiles.  Computed when a block moves to another unit: the 64-bit divisions
+// took longer than a tile's arithmetic when every tile repeated them (2^25
+// floats, 456 units: 29.4 us, now 25.1).
+struct inner_unit { size_t j, base, count, tiles; };
+template <class T> __device__ __forceinline__ inner_unit inner_unit_of(const inner_tma_shape& sh, size_t u)
 {
-  const size_t r0 = (u % sh.splits) * sh.seg;
-  const size_t r1 = (r0 + sh.seg < sh.rows) ? r0 + sh.seg : sh.rows;
-  return (r1 - r0 + inner_tile<T>() - 1) / inner_tile<T>();
+  inner_unit w;
+  w.j = u / sh.splits;
+  const size_t r0 = (u - w.j * sh.splits) * sh.seg;
+  w.base = w.j * sh.rows + r0;
+  w.count = sh.rows - r0 < sh.seg ? sh.rows - r0 : sh.seg;
+  w.tiles = (w.count + inner_tile<T>() - 1) / inner_tile<T>();
+  return w;
 }
 
 // NT = 1 folds x; NT = 2 folds x*y (float product rounded, as NT2's X*Y).
@@ -152,13 +164,12 @@ __global__ void __launch_bounds__(256) k_inner_tma(const T* __restrict__ x, cons
   if (blockIdx.x < sh.units) {
     // while the previous grid drains, have the L2 fetch the first STAGES tiles
     // of this block's first unit (one prefetch per 128-byte line)
-    const size_t u = blockIdx.x, j = u / sh.splits, r0 = (u % sh.splits) * sh.seg;
-    const size_t rend = (r0 + sh.seg < sh.rows) ? r0 + sh.seg : sh.rows;
-    const size_t span = (rend - r0 < (size_t)STAGES * TILE) ? rend - r0 : (size_t)STAGES * TILE;
+    const inner_unit w = inner_unit_of<T>(sh, blockIdx.x);
+    const size_t span = (w.count < (size_t)STAGES * TILE) ? w.count : (size_t)STAGES * TILE;
     const size_t lines = (span * sizeof(T) + 127) / 128;
     for (size_t q = threadIdx.x; q < lines; q += blockDim.x) {
-      nt2cuda::mem::prefetch_l2(reinterpret_cast<const char*>(x + j * sh.rows + r0) + q * 128);
-      if constexpr (NT == 2) nt2cuda::mem::prefetch_l2(reinterpret_cast<const char*>(y + j * sh.rows + r0) + q * 128);
+      nt2cuda::mem::prefetch_l2(reinterpret_cast<const char*>(x + w.base) + q * 128);
+      if constexpr (NT == 2) nt2cuda::mem::prefetch_l2(reinterpret_cast<const char*>(y + w.base) + q * 128);
     }
   }
   nt2cuda::mem::pdl_begin();
@@ -177,24 +188,32 @@ __global__ void __launch_bounds__(256) k_inner_tma(const T* __restrict__ x, cons
   // producer state (thread 0): next tile to issue
   size_t pu = blockIdx.x, pt = 0;
   uint32_t issued = 0;
+  inner_unit pw{};
+  if (pu < sh.units) pw = inner_unit_of<T>(sh, pu);
   auto produce = [&](int s) {
-    const size_t j = pu / sh.splits, r0 = (pu % sh.splits) * sh.seg + pt * (size_t)TILE;
-    const size_t rend = ((pu % sh.splits) * sh.seg + sh.seg < sh.rows) ? (pu % sh.splits) * sh.seg + sh.seg : sh.rows;
-    const uint32_t cnt = (uint32_t)((rend - r0) < (size_t)TILE ? (rend - r0) : (size_t)TILE);
+    const size_t off = pt * (size_t)TILE;
+    const uint32_t cnt = (uint32_t)((pw.count - off) < (size_t)TILE ? (pw.count - off) : (size_t)TILE);
     const uint32_t bytes = cnt * (uint32_t)sizeof(T);
     tma::mbar_arrive_expect_tx(&bar[s], bytes * NT);
     if (!(pu == sh.fail_unit && pt == 0)) {
-      tma::bulk_g2s(buf + (size_t)(s * NT) * TILE, x + j * sh.rows + r0, bytes, &bar[s]);
-      if constexpr (NT == 2) tma::bulk_g2s(buf + (size_t)(s * NT + 1) * TILE, y + j * sh.rows + r0, bytes, &bar[s]);
+      tma::bulk_g2s(buf + (size_t)(s * NT) * TILE, x + pw.base + off, bytes, &bar[s]);
+      if constexpr (NT == 2) tma::bulk_g2s(buf + (size_t)(s * NT + 1) * TILE, y + pw.base + off, bytes, &bar[s]);
     }
     ++issued;
-    if (++pt == inner_unit_tiles<T>(sh, pu)) { pt = 0; pu += gridDim.x; }
+    if (++pt == pw.tiles) {
+      pt = 0;
+      pu += gridDim.x;
+      if (pu < sh.units) pw = inner_unit_of<T>(sh, pu);
+    }
   };
   if (threadIdx.x == 0)
     for (int s = 0; s < STAGES && pu < sh.units; ++s) produce(s);
 
   size_t cu = blockIdx.x, ct = 0;
   uint32_t iter = 0;
+  inner_unit w{};
+  if (cu < sh.units) w = inner_unit_of<T>(sh, cu);
+  block_acc<Op, T, term<T>> ba;
   S a[V];
 #pragma unroll
   for (int l = 0; l < V; ++l) a[l] = Op::template init<T>();
@@ -210,14 +229,22 @@ __global__ void __launch_bounds__(256) k_inner_tma(const T* __restrict__ x, cons
       __syncthreads();
       return;
     }
-    const size_t j = cu / sh.splits;
-    const size_t seg0 = (cu % sh.splits) * sh.seg;
-    const size_t rend = (seg0 + sh.seg < sh.rows) ? seg0 + sh.seg : sh.rows;
-    const size_t r0 = seg0 + ct * (size_t)TILE;
-    const int cnt = (int)((rend - r0) < (size_t)TILE ? (rend - r0) : (size_t)TILE);
+    const size_t left = w.count - ct * (size_t)TILE;
+    const int cnt = (int)(left < (size_t)TILE ? left : (size_t)TILE);
     const T* tx = buf + (size_t)(s * NT) * TILE;
     const T* ty = buf + (size_t)(s * NT + (NT == 2 ? 1 : 0)) * TILE;
-    for (int e = threadIdx.x * V; e < cnt; e += 256 * V) {
+    constexpr bool BLK = NT == 1 && block_acc<Op, T, term<T>>::value;
+    if constexpr (BLK) {
+      if (cnt == TILE) {                               // a thread's values of the tile form a block
+        constexpr int Q = TILE / (256 * V);
+        T blk[Q * V];
+#pragma unroll
+        for (int q = 0; q < Q; ++q)
+          *reinterpret_cast<uint4*>(blk + q * V) = *reinterpret_cast<const uint4*>(tx + (q * 256 + threadIdx.x) * V);
+        ba.add(a[0], blk);
+      }
+    }
+    for (int e = BLK && cnt == TILE ? cnt : threadIdx.x * V; e < cnt; e += 256 * V) {
       T xv[V];
       *reinterpret_cast<uint4*>(xv) = *reinterpret_cast<const uint4*>(tx + e);
       if constexpr (NT == 2) {
@@ -225,8 +252,8 @@ __global__ void __launch_bounds__(256) k_inner_tma(const T* __restrict__ x, cons
         *reinterpret_cast<uint4*>(yv) = *reinterpret_cast<const uint4*>(ty + e);
 #pragma unroll
         for (int l = 0; l < V; ++l) Op::add(a[l], math::mul(xv[l], yv[l]));
-      } else if constexpr (has_block_add<Op>::value) {
-        Op::add_block(a[0], xv);                       // var/stdev: one merge per V values
+      } else if constexpr (BLK) {
+        ba.add(a[0], xv);
       } else {
 #pragma unroll
         for (int l = 0; l < V; ++l) Op::add(a[l], xv[l]);
@@ -237,7 +264,9 @@ __global__ void __launch_bounds__(256) k_inner_tma(const T* __restrict__ x, cons
       tma::fence_proxy_async();
       produce(s);
     }
-    if (++ct == inner_unit_tiles<T>(sh, cu)) {         // unit complete: merge and emit
+    if (++ct == w.tiles) {                             // unit complete: merge and emit
+      const size_t j = w.j;
+      if constexpr (BLK) ba.flush(a[0]);
       S t = a[0];
 #pragma unroll
       for (int l = 1; l < V; ++l) t = Op::merge(t, a[l]);
@@ -257,9 +286,8 @@ __global__ void __launch_bounds__(256) k_inner_tma(const T* __restrict__ x, cons
           if (threadIdx.x == 0) out[j] = quiet_nan<out_of<Op, T>>();
         } else if (s_last) {
           __threadfence();
-          S m = Op::template init<T>();
-          for (size_t q = threadIdx.x; q < sh.splits; q += blockDim.x)
-            m = Op::merge(m, Op::ldcg(partials + j * sh.splits + q));
+          const size_t mine = sh.splits > threadIdx.x ? (sh.splits - threadIdx.x + blockDim.x - 1) / blockDim.x : 0;
+          S m = merge_partials<Op, T>(partials + j * sh.splits + threadIdx.x, mine, blockDim.x);
           m = block_merge<Op, T>(m, red);
           if (threadIdx.x == 0) out[j] = Op::finish(m, sh.rows);
         }
@@ -268,6 +296,7 @@ __global__ void __launch_bounds__(256) k_inner_tma(const T* __restrict__ x, cons
       for (int l = 0; l < V; ++l) a[l] = Op::template init<T>();
       ct = 0;
       cu += gridDim.x;
+      if (cu < sh.units) w = inner_unit_of<T>(sh, cu);
     }
     ++iter;
   }
@@ -420,8 +449,13 @@ cudaError_t inner_fold_tma(const T* x, const T* y, size_t rows, size_t cols, out
   inner_tma_shape sh;
   sh.rows = rows;
   sh.cols = cols;
-  sh.seg = (size_t)TILE * 16;
+  sh.seg = inner_tma_seg<T>(rows, cols, y ? 2 : 1);
   sh.splits = (rows + sh.seg - 1) / sh.seg;
+  // a stream captured before its scratch was allocated: columns of one unit each
+  if (sh.splits > 1 && rows <= (size_t)TILE * 16 && fold_scratch_barred(s, cols, cols * sh.splits, sizeof(S))) {
+    sh.seg = rows;
+    sh.splits = 1;
+  }
   sh.units = cols * sh.splits;
   sh.fail_unit = fail_unit;
   sh.wait_rounds = wait_rounds;

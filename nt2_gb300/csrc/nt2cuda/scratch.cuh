@@ -44,11 +44,30 @@ inline cudaError_t fold_scratch(cudaStream_t s, size_t ncounters, size_t npartia
   return e;
 }
 
-inline cudaError_t stream_scratch(cudaStream_t s, size_t bytes, void** out, int slot)
+inline uintptr_t scratch_key(cudaStream_t s, int slot)
 {
   int dev = 0;
   cudaGetDevice(&dev);
-  uintptr_t key = (reinterpret_cast<uintptr_t>(s) * 64u + (uintptr_t)dev) * 4u + (uintptr_t)slot;
+  return (reinterpret_cast<uintptr_t>(s) * 64u + (uintptr_t)dev) * 4u + (uintptr_t)slot;
+}
+
+// Whether a fold's buffers could not be had now: they would have to be
+// allocated, and the stream is being captured.
+inline bool fold_scratch_barred(cudaStream_t s, size_t ncounters, size_t npartials, size_t partial_bytes)
+{
+  {
+    scratch_pool& P = global_scratch_pool();
+    const uintptr_t k0 = scratch_key(s, 0), k2 = scratch_key(s, 2);
+    std::lock_guard<std::mutex> g(P.m);
+    if (P.by_key[k0].bytes >= ncounters * sizeof(unsigned) && P.by_key[k2].bytes >= npartials * partial_bytes) return false;
+  }
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(s, &st) == cudaSuccess && st != cudaStreamCaptureStatusNone;
+}
+
+inline cudaError_t stream_scratch(cudaStream_t s, size_t bytes, void** out, int slot)
+{
+  const uintptr_t key = scratch_key(s, slot);
   scratch_pool& P = global_scratch_pool();
   std::lock_guard<std::mutex> g(P.m);
   scratch_pool::entry& e = P.by_key[key];
