@@ -41,6 +41,7 @@ inline params lookup(const char* key, size_t n, params def = params{})
 {
   if (!key) return def;
   std::lock_guard<std::mutex> g(table_mutex());
+  if (table().empty()) return def;                 // nothing tuned: no key to build
   auto it = table().find(make_key(key, n));
   return it == table().end() ? def : it->second;
 }
