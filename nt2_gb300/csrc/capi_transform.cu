@@ -208,7 +208,8 @@ nt2cuda_status bs_launch(const T* S, const T* K, const T* Tm, T r, T v, T* call,
   size_t nn = n;
   void* args[] = {(void*)&S, (void*)&K, (void*)&Tm, (void*)&r, (void*)&v, (void*)&call, (void*)&put, (void*)&nn};
   const bool vec = sizeof(T) == 4 && aligned16(S) && aligned16(K) && aligned16(Tm) && aligned16(call) && aligned16(put);
-  if (!vec) return launch_status(launch_persistent(k_blackscholes_scalar<T, CDF, P>, n, 256, waves, s, args));
+  if (!vec)
+    return launch_status(launch_persistent(k_blackscholes_scalar<T, CDF, P>, n, sizeof(T) == 8 ? f64_block(n) : 256, waves, s, args));
   if constexpr (sizeof(T) == 4) {
     size_t groups = n / 4;
     switch (unroll) {
