@@ -94,6 +94,27 @@ __device__ __forceinline__ void tensor_g2s_2d(void* dst, const CUtensorMap* map,
       : "memory");
 }
 
+// 3-D tiled load and store through a tensor map; x and the alignment as above
+__device__ __forceinline__ void tensor_g2s_3d(void* dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar)
+{
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::
+          "r"(smem_u32(dst)),
+      "l"(map), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
+      : "memory");
+}
+__device__ __forceinline__ void tensor_s2g_3d(const CUtensorMap* map, int x, int y, int z, const void* src)
+{
+  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%1, %2, %3}], [%4];" ::"l"(map), "r"(x),
+               "r"(y), "r"(z), "r"(smem_u32(src))
+               : "memory");
+}
+
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar)
+{
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
 // 2-D tiled store shared -> global through a tensor map (a bulk group of
 // this thread; complete it with bulk_commit and wait with bulk_wait*)
 __device__ __forceinline__ void tensor_s2g_2d(const CUtensorMap* map, int x, int y, const void* src)
