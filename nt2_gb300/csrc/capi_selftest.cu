@@ -173,6 +173,36 @@ template <bool ABS, bool F> __device__ __forceinline__ void x2_check_pow(uint32_
   }
 }
 
+// 28..31: as 22..25 over bases and exponents that whole warps share the range of
+// (every base normal and finite, |exponent| < 2^18), which is what the packed
+// pow's shorter form is chosen by: results all normal, astride both ends of the
+// range, next to the ends, and far past them.
+template <bool ABS, bool F> __device__ __forceinline__ void x2_check_pow_moderate(uint32_t u0, x2_report* rep)
+{
+  float a[2], b[2];
+#pragma unroll
+  for (int l = 0; l < 2; ++l) {
+    const uint32_t u = u0 + l, h = mix32(u), ex = (u >> 23) & 255u;
+    const float unit = (float)(h >> 8) * (1.0f / 16777216.0f) - 0.5f;
+    a[l] = __uint_as_float((u & (ABS ? 0x807fffffu : 0x007fffffu)) | (min(max(ex, 1u), 254u) << 23));
+    const float lg = log2f(fabsf(a[l]));
+    float t;
+    switch ((u >> 6) & 3u) {
+      case 0: t = unit * 244.0f / lg; break;
+      case 1: t = unit * 600.0f / lg; break;
+      case 2: t = ((h & 1u ? 126.5f : -126.5f) + unit * 4.0f) / lg; break;
+      default: t = (h & 1u) ? unit * 524200.0f : (float)((int)(h % 129u) - 64); break;
+    }
+    b[l] = fabsf(t) < 262144.0f ? t : unit;
+  }
+  const float2 r = ABS ? x2::pow_abs<F>(make_float2(a[0], a[1]), make_float2(b[0], b[1]))
+                       : x2::pow<F>(make_float2(a[0], a[1]), make_float2(b[0], b[1]));
+  const float s0 = ABS ? math::pow_abs<F>(a[0], b[0]) : math::pow<F>(a[0], b[0]);
+  const float s1 = ABS ? math::pow_abs<F>(a[1], b[1]) : math::pow<F>(a[1], b[1]);
+  if (!same(r.x, s0)) record(rep, u0);
+  if (!same(r.y, s1)) record(rep, u0 + 1);
+}
+
 // 26, 27: cbrt, unfused and fused
 __device__ __forceinline__ void x2_check_cbrt(bool fused, uint32_t u0, x2_report* rep)
 {
@@ -205,6 +235,10 @@ __global__ void __launch_bounds__(256) k_x2_check(int which, uint64_t pairs, x2_
     else if (which == 23) x2_check_pow<false, true>((uint32_t)(2 * p), rep);
     else if (which == 24) x2_check_pow<true, false>((uint32_t)(2 * p), rep);
     else if (which == 25) x2_check_pow<true, true>((uint32_t)(2 * p), rep);
+    else if (which == 28) x2_check_pow_moderate<false, false>((uint32_t)(2 * p), rep);
+    else if (which == 29) x2_check_pow_moderate<false, true>((uint32_t)(2 * p), rep);
+    else if (which == 30) x2_check_pow_moderate<true, false>((uint32_t)(2 * p), rep);
+    else if (which == 31) x2_check_pow_moderate<true, true>((uint32_t)(2 * p), rep);
     else x2_check_cbrt(which == 27, (uint32_t)(2 * p), rep);
   }
 }
@@ -285,7 +319,7 @@ extern "C" nt2cuda_status nt2cuda_selftest_x2(int which, unsigned long long* mis
                                               nt2cuda_stream stream)
 {
   NT2CUDA_NVTX_RANGE;
-  if (which < 0 || which > 27 || !mismatches) return NT2CUDA_ERR_ARG;
+  if (which < 0 || which > 31 || !mismatches) return NT2CUDA_ERR_ARG;
   cudaStream_t s = as_stream(stream);
   x2_report* rep = nullptr;
   cudaError_t e = cudaMalloc(&rep, sizeof(x2_report));

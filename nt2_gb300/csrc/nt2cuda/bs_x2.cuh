@@ -547,6 +547,117 @@ template <bool F, bool PLAIN> __device__ __forceinline__ float2 pow_abs_core(flo
   }
 }
 
+// pow for a pair of ordinary arguments (|a0| normal and finite, |a1| < 2^18).
+// The per-lane integer and select work of
+// pow_abs_core is what bound it (58 of 113 instructions an element on the ALU
+// pipe), so here
+//  * the search for the table index is one comparison with the threshold of the
+//    mantissa's top five bits (a bin of 1/64 holds at most one), and A[i],
+//    B[i/2], 1/A[i] and -i/16 come with one 16-byte read;
+//  * the quotient by A[i] is Markstein's correction from the tabulated 1/A[i];
+//  * floor(16 x)/16 is two packed fma, the first rounding x*16 + 1.5*2^23 down
+//    (exact products; |16 x| < 2^22 for every x whose result is kept);
+//  * the small integers come from and go to floats through the same sum;
+//  * 2^i adds to the exponent where the warp's results are all normal; else the
+//    range selections and the two-step scaling follow.
+// 2^24 pairs, a0 in [0, 100], a1 in [-10, 10]: 74.3 us before, 59.0 now.
+static __device__ const uint2 kPowBin[32] = {   // {last mantissa pattern past the bin's threshold, index/2 before it}
+  {0x00000000u, 8u}, {0x3f05aac3u, 7u}, {0x00000000u, 7u}, {0x00000000u, 7u}, {0x3f11c3d3u, 6u}, {0x00000000u, 6u}, {0x00000000u, 6u}, {0x3f1ef532u, 5u},
+  {0x00000000u, 5u}, {0x00000000u, 5u}, {0x00000000u, 5u}, {0x3f2d583fu, 4u}, {0x00000000u, 4u}, {0x00000000u, 4u}, {0x00000000u, 4u}, {0x3f3d08a4u, 3u},
+  {0x00000000u, 3u}, {0x00000000u, 3u}, {0x00000000u, 3u}, {0x3f4e248cu, 2u}, {0x00000000u, 2u}, {0x00000000u, 2u}, {0x00000000u, 2u}, {0x00000000u, 2u},
+  {0x3f60ccdfu, 1u}, {0x00000000u, 1u}, {0x00000000u, 1u}, {0x00000000u, 1u}, {0x00000000u, 1u}, {0x3f75257cu, 0u}, {0x00000000u, 0u}, {0x00000000u, 0u}};
+static __device__ const uint4 kPowEntry[9] = {  // A[i], B[i/2], 1/A[i], -i/16 for i = 0, 2, ... 16
+  {0x3f800000u, 0x00000000u, 0x3f800000u, 0x00000000u}, {0x3f6ac0c7u, 0xb1c116deu, 0x3f8b95c2u, 0xbe000000u},
+  {0x3f5744fdu, 0xb254a58au, 0x3f9837f0u, 0xbe800000u}, {0x3f45672au, 0x318aa837u, 0x3fa5fed7u, 0xbec00000u},
+  {0x3f3504f3u, 0x324fe77au, 0x3fb504f3u, 0xbf000000u}, {0x3f25fed7u, 0xb2ac9d5eu, 0x3fc5672au, 0xbf200000u},
+  {0x3f1837f0u, 0x32a31b71u, 0x3fd744fdu, 0xbf400000u}, {0x3f0b95c2u, 0xb1e0aba1u, 0x3feac0c7u, 0xbf600000u},
+  {0x3f000000u, 0x00000000u, 0x40000000u, 0xbf800000u}};
+__device__ __forceinline__ float2 fma_down(float2 a, float2 b, float2 c)
+{
+  float2 r;
+  asm("{.reg .b64 a, b, c, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 c, {%6, %7};\n\t"
+      "fma.rm.f32x2 d, a, b, c;\n\tmov.b64 {%0, %1}, d;}"
+      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return r;
+}
+__device__ __forceinline__ float2 pow_reduc_small(float2 x)
+{
+  return fma(fma_down(splat(16.0f), x, splat(kRound)), splat(0.0625f), splat(-0.0625f * kRound));
+}
+template <bool F> __device__ __forceinline__ float2 pow_ordinary(float2 a0, float2 a1)
+{
+  using C = math::powc<float>;
+  constexpr uint32_t P1[4] = {0xbe2a61b2u, 0x3e4d2fa3u, 0xbe800015u, 0x3eaaaaa3u};   // math::pow1
+  constexpr uint32_t P2[4] = {0x3c1a49bcu, 0x3d634d38u, 0x3e75fde1u, 0x3f317218u};   // math::pow2
+  const float a[2] = {a0.x, a0.y};
+  float xs[2], es[2];
+  uint4 t[2];
+#pragma unroll
+  for (int l = 0; l < 2; ++l) {
+    const uint32_t b = __float_as_uint(a[l]) & 0x7fffffffu, m = (b & 0x007fffffu) | 0x3f000000u;
+    const uint2 bin = __ldg(&kPowBin[(b >> 18) & 31u]);
+    t[l] = __ldg(&kPowEntry[bin.y + (m <= bin.x ? 1u : 0u)]);
+    xs[l] = __uint_as_float(m);
+    es[l] = __uint_as_float((b >> 23) + (0x4b400000u - 126u));                       // e + kRound
+  }
+  const float2 A = make_float2(fbits(t[0].x), fbits(t[1].x)), rA = make_float2(fbits(t[0].z), fbits(t[1].z));
+  float2 x = sub(make_float2(xs[0], xs[1]), A);
+  x = sub(x, make_float2(fbits(t[0].y), fbits(t[1].y)));
+  const float2 q = mul(x, rA);
+  x = fma(fma(make_float2(-A.x, -A.y), q, x), rA, q);
+  float2 z = mul(x, x);
+  float2 w = mul_r(mul(z, x), horner<F>(x, P1));
+  w = madd<F>(splat(-0.5f), z, w);
+  w = madd<F>(splat(C::bits(C::log2_em1)), w, w);
+  z = madd<F>(splat(C::bits(C::log2_em1)), x, w);
+  z = add(z, x);
+  w = add(sub(make_float2(es[0], es[1]), splat(kRound)), make_float2(fbits(t[0].w), fbits(t[1].w)));   // e - i/16
+  const float2 ya = pow_reduc_small(a1);
+  const float2 yb = sub(a1, ya);
+  float2 W = madd<F>(z, a1, mul_r(w, yb));
+  float2 Wa = pow_reduc_small(W);
+  float2 Wb = sub(W, Wa);
+  W = madd<F>(w, ya, Wa);
+  Wa = pow_reduc_small(W);
+  const float2 u = sub(W, Wa);
+  W = add(Wb, u);
+  Wb = pow_reduc_small(W);
+  const float2 k = fma(splat(16.0f), add(Wa, Wb), splat(kRound));                    // 16 (Wa + Wb) + kRound
+  Wb = sub(W, Wb);
+  const float2 Wm = sub(Wb, splat(0.0625f));
+  const bool up[2] = {Wb.x > 0.0f, Wb.y > 0.0f};
+  Wb = make_float2(up[0] ? Wm.x : Wb.x, up[1] ? Wm.y : Wb.y);
+  z = mul(horner<F>(Wb, P2), Wb);
+  const uint32_t kb[2] = {__float_as_uint(k.x), __float_as_uint(k.y)};
+  int i[2];
+  float wt[2];
+#pragma unroll
+  for (int l = 0; l < 2; ++l) {
+    const int e = (int)(kb[l] - (up[l] ? 0x4b3fffffu : 0x4b400000u));
+    i[l] = (e + 15 + (e > 0 ? 1 : 0)) >> 4;                                          // e > 0 ? e/16 + 1 : e/16
+    wt[l] = math::pow_a(0.0f, (int)min((unsigned)(i[l] * 16 - e), 16u));
+  }
+  w = make_float2(wt[0], wt[1]);
+  z = madd<F>(w, z, w);
+  // z is in [1/2, 1]: normal results for -125 < i < 127.  Where |W| is past 2^18
+  // the sums above are off, and far past both limits of k below.
+  const bool normal = (unsigned)(i[0] + 124) <= 250u && (unsigned)(i[1] + 124) <= 250u;
+  if (__all_sync(__activemask(), normal))
+    return make_float2(__uint_as_float(__float_as_uint(z.x) + ((uint32_t)i[0] << 23)),
+                       __uint_as_float(__float_as_uint(z.y) + ((uint32_t)i[1] << 23)));
+  const float2 wl = sub(k, splat(kRound));
+  const float inf = __int_as_float(0x7f800000);
+  z = pow_ldexp(z, min(max(i[0], -2048), 2048), min(max(i[1], -2048), 2048));
+  z.x = wl.x > C::bits(C::large) ? inf : (wl.x < C::bits(C::low) ? 0.0f : z.x);
+  z.y = wl.y > C::bits(C::large) ? inf : (wl.y < C::bits(C::low) ? 0.0f : z.y);
+  return z;
+}
+__device__ __forceinline__ bool pow_moderate(float a0, float a1, bool pos)
+{
+  const uint32_t b = pos ? __float_as_uint(a0) : (__float_as_uint(a0) & 0x7fffffffu);
+  return b - 0x00800000u < 0x7f000000u && fabsf(a1) < 262144.0f;
+}
+
 // |a0| normal and finite, a1 finite (pos: a0 also positive, where pow is pow_abs)
 __device__ __forceinline__ bool pow_plain(float a0, float a1, bool pos)
 {
@@ -556,6 +667,8 @@ __device__ __forceinline__ bool pow_plain(float a0, float a1, bool pos)
 
 template <bool F> __device__ __forceinline__ float2 pow_abs(float2 a0, float2 a1)
 {
+  if (__all_sync(__activemask(), pow_moderate(a0.x, a1.x, false) && pow_moderate(a0.y, a1.y, false)))
+    return pow_ordinary<F>(a0, a1);
   if (__all_sync(__activemask(), pow_plain(a0.x, a1.x, false) && pow_plain(a0.y, a1.y, false)))
     return pow_abs_core<F, true>(a0, a1);
   return pow_abs_core<F, false>(a0, a1);
@@ -563,6 +676,8 @@ template <bool F> __device__ __forceinline__ float2 pow_abs(float2 a0, float2 a1
 
 template <bool F> __device__ __forceinline__ float2 pow(float2 a0, float2 a1)
 {
+  if (__all_sync(__activemask(), pow_moderate(a0.x, a1.x, true) && pow_moderate(a0.y, a1.y, true)))
+    return pow_ordinary<F>(a0, a1);
   if (__all_sync(__activemask(), pow_plain(a0.x, a1.x, true) && pow_plain(a0.y, a1.y, true)))
     return pow_abs_core<F, true>(a0, a1);
   float2 z = pow_abs_core<F, false>(a0, a1);

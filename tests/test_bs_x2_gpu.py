@@ -74,6 +74,19 @@ def test_two_lane_pow_matches_one_lane(gpu, cuda_lib, which, name):
     assert n.value == 0, (name, n.value, [hex(first[i]) for i in range(min(8, n.value))])
 
 
+@pytest.mark.parametrize("which,name", [(28, "pow"), (29, "pow, fused"), (30, "pow_abs"), (31, "pow_abs, fused")])
+def test_two_lane_pow_of_ordinary_warps_matches_one_lane(gpu, cuda_lib, which, name):
+    """Where a warp's bases are all normal and its exponents below 2^18, pow and pow_abs
+    take a shorter form: over every base of that kind, with exponents whose results are
+    normal, next to the ends of the range, astride them and far past them, both lanes give
+    the one-lane bits."""
+    n = C.c_ulonglong(99)
+    first = (C.c_uint32 * 8)()
+    st = cuda_lib.nt2cuda_selftest_x2(which, C.byref(n), first, torch.cuda.current_stream().cuda_stream)
+    assert st == 0
+    assert n.value == 0, (name, n.value, [hex(first[i]) for i in range(min(8, n.value))])
+
+
 @pytest.mark.parametrize("which,name", [(26, "cbrt"), (27, "cbrt, fused")])
 def test_two_lane_cbrt_is_bit_exact_over_every_float(gpu, cuda_lib, which, name):
     """FP32 cbrt nodes run two lanes per packed instruction, the Newton step's division by a
