@@ -35,13 +35,14 @@ template <class E> bool expr_aligned(const E& e)
 // 44 us with segments of 16384, 10.5 with 2432 of them), but never below eight
 // loads a lane, and at most kInnerSplits to a column, as one warp merges them.
 // The cut depends on the table's shape alone: results are reproducible.
-// (var/stdev of doubles: 1216, 8 a SM, as merging their partials takes longer.)
-constexpr size_t kInnerUnits = 3648, kInnerUnitsScalar = 2432, kInnerUnitsFramed = 1216, kInnerSplits = 2432;
+// (var/stdev of doubles: 16 a SM in either case, what their 128 registers leave
+// room for; 70000 x 111: 46.9 us with 8, 40.7 with 16, 41.6 with 24.)
+constexpr size_t kInnerUnits = 3648, kInnerUnitsScalar = 2432, kInnerSplits = 2432;
 constexpr size_t kInnerWhole = 4096;     // 16-byte groups of the longest column folded whole under capture
 template <class Op, class T> inline size_t inner_seg(size_t rows, size_t cols, bool vec)
 {
   const size_t lanes = vec ? 32 * (16 / sizeof(T)) : 32;
-  const size_t units = warp_framed<Op, T>::value ? kInnerUnitsFramed : (vec ? kInnerUnits : kInnerUnitsScalar);
+  const size_t units = vec && !warp_framed<Op, T>::value ? kInnerUnits : kInnerUnitsScalar;
   size_t splits = (units + cols / 2) / cols;              // rounded: half a segment more or less a column
   if (splits < 1) splits = 1;
   if (splits > kInnerSplits) splits = kInnerSplits;
