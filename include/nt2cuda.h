@@ -394,7 +394,8 @@ nt2cuda_status nt2cuda_set_fold_path(int path);
  *  modules/boost/simd/base/include/boost/simd/reduction/functions/{sum,maximum,minimum,prod}.hpp)
  * FP32 sums accumulate compensated unless NT2CUDA_RED_PLAIN is set; var and
  * stdev normalise by n - 1 (NT2's w = 0; by n with NT2CUDA_RED_VAR_N) and are
- * computed in one pass (Welford updates, Chan merges).  max and min skip NaNs;
+ * computed in one pass (block updates or, for doubles, exact fixed-point sums;
+ * Chan merges).  max and min skip NaNs;
  * a fold of zero elements gives NT2's neutral value (0, 1, -FLT_MAX, FLT_MAX). */
 enum {
   NT2CUDA_RED_SUM = 0, NT2CUDA_RED_ASUM1 = 1, NT2CUDA_RED_ASUM2 = 2, NT2CUDA_RED_NORM2 = 3,
