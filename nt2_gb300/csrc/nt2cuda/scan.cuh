@@ -692,13 +692,15 @@ __global__ void __launch_bounds__(256, (scan_min_blocks<Op, T>::value)) k_scan_i
 // thread's 16-byte accesses to its own row meet no bank twice).
 //
 // Instead of a look-back from inclusive prefix to inclusive prefix, every block
-// folds the aggregates of all the column's tiles before its own: between one of
-// its tiles and the next about one from each other block, a gather of 8-byte
-// words and no chain of waits.  The fold is fixed by the tiles' places: lane l
-// takes the column's tiles l, l + 32, ... in order, and the lanes meet in a
-// butterfly; so results do not depend on timing.  The word is the tile's compensated pair; all ones says that it is not
-// there yet (scratch is set to that; no pair has these bits, as a NaN sum's
-// compensation is stored as 0), 0xff..fe that a wait for it ran out.
+// adds up the aggregates of all the column's tiles before its own: between one of
+// its tiles and the next about one from each other block, a gather of 64 bytes
+// each and no chain of waits.  The sum is exact, as in the look-back of the other
+// columns: a tile publishes its compensated pair as seven signed digits of 48
+// bits (units of 2^-149, so every finite float and any sum of 2^31 of them), and
+// digits add as integers, whatever the order.  A float fold of the pairs would
+// lose what cancels between tiles, and overflow where a partial sum taken out of
+// order exceeds every prefix.  A word's top two bits are 0; scratch starts as
+// bytes of 0x7f (not there yet), kStreamFailed stands for a wait that ran out.
 //
 // Tiles are handed out by a ticket in order, and a block folds and publishes a
 // tile as soon as it has arrived, whatever its earlier tiles wait for; so no
@@ -706,34 +708,132 @@ __global__ void __launch_bounds__(256, (scan_min_blocks<Op, T>::value)) k_scan_i
 // and no block needs another to be resident.
 //
 // Roles, each a loop over the block's tiles with a barrier per stage between
-// them: load/store (one thread), fold (12 warps), publish (1), gather (1: the
+// them: load/store (one thread), fold (12 warps), publish (1), gather (5: the
 // tile's prefix), rescan (12).  (The 12 warps
 // fold and rescan with 26 instructions an element between them, two thirds of
-// the SM's issue slots at full bandwidth, so the one gathering warp's work is
-// kept short: exact 320-bit sums, or a warp scan per 32 words, took 120 to 250 us.)
-// 2^26 floats: 98 to 101 us, 79% of a copy of the same bytes (79 us); the
-// two-pass tiles with the look-back 151.  10^5 x 30: 14.9 against 18.9.
+// the SM's issue slots at full bandwidth, so the gathering warps' work is
+// kept short: four lanes share a tile's digits, so that a tile is one 16-byte
+// load and four additions in each, and the pair is made from the digits as floats.
+// The warps share the 152 or so tiles of a gather, so that its loads are in flight
+// at once: 2^26 floats 106 us with one or two warps, 102.6 with three of seven loads
+// a lane, 100.1 with five of four.)
+// 2^26 floats: 100 us, 79% of a copy of the same bytes (79 us); the two-pass tiles
+// with the look-back 151.  200000 x 200: 64.5 against 90.
 constexpr int kStreamWarps = 12, kStreamStages = 4;
 constexpr int kStreamRows = 32 * kStreamWarps;
 constexpr size_t kStreamTile = (size_t)kStreamRows * 32;            // floats
-constexpr int kStreamThreads = 32 * (2 * kStreamWarps + 3);
+constexpr int kStreamGather = 5, kStreamLoads = 4;                  // gathering warps, loads a lane has in flight
+constexpr int kStreamThreads = 32 * (2 * kStreamWarps + 2 + kStreamGather);
 constexpr size_t kStreamSmem = kStreamStages * kStreamTile * sizeof(float) + 1024;   // + alignment to the swizzle's 1 KB
-constexpr unsigned long long kStreamEmpty = ~0ull, kStreamFailed = ~1ull;
+constexpr int kStreamWords = 8;                                     // of a tile's aggregate
+constexpr unsigned long long kStreamEmpty = 0x7f7f7f7f7f7f7f7full, kStreamFailed = 0x4000000000000000ull;
+constexpr unsigned long long kStreamBias = 1ull << 50;              // makes a published digit positive
 
 struct stream_shape {
   size_t rows, cols, tiles_per_col, tiles;
   uint32_t wait_rounds;            // of the block's own barriers
 };
 
-// One float pair as the word other blocks read.
-__device__ __forceinline__ unsigned long long stream_word(const fold::acc<float>& a)
+// Digit j (48 bits, weight 2^(48 j - 149)) of a finite float, with its sign.
+__device__ __forceinline__ long long stream_digit(float f, int j)
 {
-  return ((unsigned long long)__float_as_uint(isfinite(a.s) ? a.c : 0.f) << 32) | __float_as_uint(a.s);
+  const unsigned u = __float_as_uint(f), be = (u >> 23) & 255u;
+  const unsigned long long m = (u & 0x7fffffu) | (be ? 0x800000u : 0u);
+  const int p = (int)(be ? be - 1u : 0u) - 48 * j;                  // m's lowest bit in the digit
+  long long d = 0;
+  if (p >= 0 && p < 48) d = (long long)((m << p) & 0xffffffffffffull);
+  if (p < 0 && p > -24) d = (long long)(m >> -p);
+  return u >> 31 ? -d : d;
+}
+// Non-finite values a sum holds: 1 for +Inf, 2 for -Inf, 4 for NaN.
+__device__ __forceinline__ unsigned stream_special(float f)
+{
+  return isfinite(f) ? 0u : (f != f ? 4u : (f > 0.f ? 1u : 2u));
+}
+// Word j of a tile's aggregate: digits 0 to 6, then the non-finite values.  (The
+// pair's value is s and c, or s alone once s is not finite: fold::result.)
+__device__ __forceinline__ unsigned long long stream_word(const fold::acc<float>& a, int j)
+{
+  const float c = isfinite(a.s) ? a.c : 0.f;
+  if (j == 7) return stream_special(a.s) | stream_special(c);
+  return (unsigned long long)((isfinite(a.s) ? stream_digit(a.s, j) : 0) + (isfinite(c) ? stream_digit(c, j) : 0)) + kStreamBias;
+}
+__device__ __forceinline__ bool stream_missing(ulonglong2 w) { return ((w.x | w.y) >> 62) != 0ull; }
+
+// The digits of a column's running sum, as the lanes of a warp hold them: lane l
+// digits 2 (l % 4) and 2 (l % 4) + 1, the latter 0 in lane 3.
+struct stream_sum { long long x, y; };
+// Each lane's own sum over the lanes of its kind.
+__device__ __forceinline__ stream_sum stream_reduce(stream_sum a)
+{
+#pragma unroll
+  for (int off = 4; off < 32; off <<= 1) {
+    a.x += __shfl_xor_sync(0xffffffffu, a.x, off);
+    a.y += __shfl_xor_sync(0xffffffffu, a.y, off);
+  }
+  return a;
+}
+// Carry: digits are left within 2^47 + 1 of zero (the top one holds the rest), so
+// that the topmost that is not 0 has the sum's sign and at least half its size.
+__device__ __forceinline__ void stream_carry(stream_sum& r)
+{
+  const int j = threadIdx.x & 3;
+  constexpr long long half = 1ll << 47;
+#pragma unroll
+  for (int pass = 0; pass < 2; ++pass) {
+    const long long c0 = j < 3 ? (r.x + half) >> 48 : 0;
+    r.x -= c0 * (1ll << 48);
+    r.y += c0;
+    const long long c1 = (r.y + half) >> 48;
+    r.y -= c1 * (1ll << 48);
+    const long long in = __shfl_up_sync(0xffffffffu, c1, 1, 4);
+    r.x += j > 0 ? in : 0;
+  }
+}
+// The sum as a float pair: its three top digits as six floats of 24 bits each
+// (the last, past the pair's 48 bits, left out), added from the lowest up without
+// rounding errors, which meet in c.  The values are multiples of 2^-149, so a
+// subnormal pair is exact.
+__device__ __forceinline__ fold::acc<float> stream_pair(const stream_sum& r, unsigned special)
+{
+  using math::add;
+  using math::sub;
+  const int lane = threadIdx.x & 31;
+  if (special)
+    return fold::acc<float>{(special & 4u) || special == 3u ? nan_value<float>() : __int_as_float(special == 1u ? 0x7f800000 : (int)0xff800000u), 0.f};
+  const long long x = __shfl_sync(0xffffffffu, r.x, (lane >> 1) & 3), y = __shfl_sync(0xffffffffu, r.y, (lane >> 1) & 3);
+  const long long d = lane < 7 ? ((lane & 1) ? y : x) : 0;           // lane l: digit l
+  const unsigned nz = __ballot_sync(0xffffffffu, d != 0);
+  if (nz == 0u) return fold::acc<float>{0.f, 0.f};
+  const int t = 31 - __clz((int)nz);
+  float f[6];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const long long v = __shfl_sync(0xffffffffu, d, t >= i ? t - i : 31);
+    const int h = (int)((v + (1ll << 23)) >> 24);
+    f[2 * i] = (float)h;
+    f[2 * i + 1] = (float)(int)(v - (long long)h * (1ll << 24));
+  }
+  const float f0 = f[0] * 0x1p48f, f1 = f[1] * 0x1p24f, f3 = f[3] * 0x1p-24f, f4 = f[4] * 0x1p-48f;
+  const float s3 = add(f3, f4), e3 = sub(f4, sub(s3, f3));
+  const float s2 = add(f[2], s3), e2 = sub(s3, sub(s2, f[2]));
+  const float s1 = add(f1, s2), e1 = sub(s2, sub(s1, f1));
+  const float s0 = add(f0, s1), e0 = sub(s1, sub(s0, f0));
+  const float c = add(e0, add(e1, add(e2, e3)));
+  const int n = 48 * t - 173, n0 = n >> 1;                           // f[2]'s unit is 2^n
+  const float p0 = __int_as_float((127 + n0) << 23), p1 = __int_as_float((127 + n - n0) << 23);
+  return fold::acc<float>{s0 * p0 * p1, c * p0 * p1};
 }
 __device__ __forceinline__ unsigned long long stream_ld(const unsigned long long* p)
 {
   unsigned long long v;
   asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ ulonglong2 stream_ld2(const unsigned long long* p)
+{
+  ulonglong2 v;
+  asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p) : "memory");
   return v;
 }
 __device__ __forceinline__ void stream_st(unsigned long long* p, unsigned long long v)
@@ -765,11 +865,13 @@ __global__ void __launch_bounds__(kStreamThreads, 1)
   constexpr uint32_t TBYTES = (uint32_t)(kStreamTile * sizeof(float));
   constexpr unsigned long long END = ~0ull;
   // one barrier of each kind per stage; tile i of the block is at stage i % N, phase (i / N) & 1
-  __shared__ __align__(8) uint64_t full[N], folded[N], published[N], prefixed[N], done[N];
+  __shared__ __align__(8) uint64_t full[N], folded[N], published[N], shared_out[N], prefixed[N], done[N];
   __shared__ unsigned long long s_tile[N];                        // the stage's tile
   __shared__ unsigned s_k[N], s_col[N];                           // its place in its column
   __shared__ S s_row[N][kStreamRows];                             // the rows' prefixes within their warp
   __shared__ S s_tot[N][W], s_ex[N][W], s_pre[N][W];              // the warps' totals; prefixes in the tile, the column
+  __shared__ stream_sum s_share[N][kStreamGather - 1][4];         // the other gathering warps' digits, and what they met
+  __shared__ unsigned s_flags[N][kStreamGather - 1];
   __shared__ int s_bad[N];                                        // an aggregate before the tile is not to be had
   __shared__ int s_abort;                                         // a barrier wait of this block ran out
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -779,6 +881,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1)
       tma::mbar_init(&full[q], 1);
       tma::mbar_init(&folded[q], W);
       tma::mbar_init(&published[q], 1);
+      tma::mbar_init(&shared_out[q], kStreamGather - 1);
       tma::mbar_init(&prefixed[q], 1);
       tma::mbar_init(&done[q], W);
     }
@@ -882,7 +985,8 @@ __global__ void __launch_bounds__(kStreamThreads, 1)
         const S o = Op::shfl_from(c, lane >= d ? lane - d : 0);
         if (lane >= d) c = Op::merge(o, c);
       }
-      if (lane == W - 1) stream_st(agg + t, stream_word(c));
+      const S tile = Op::shfl_from(c, W - 1);
+      if (lane < kStreamWords) stream_st(agg + t * kStreamWords + lane, stream_word(tile, lane));
       S ex = Op::shfl_from(c, lane > 0 ? lane - 1 : 0);
       if (lane == 0) ex = Op::template init<float>();
       if (lane < W) s_ex[st][lane] = ex;
@@ -891,10 +995,12 @@ __global__ void __launch_bounds__(kStreamThreads, 1)
     }
   }
 
-  if (warp == 2 * W + 1) {
+  if (warp <= 2 * W + kStreamGather) {
     // -------------------------------------------------------------- gather
-    S mine = Op::template init<float>();    // this lane's fold of the column's first `groups` rounds of 32 tiles
-    unsigned groups = 0, column = 0;
+    // (each of the warps a share of the tiles; the first one puts the shares together)
+    const int gw = warp - (2 * W + 1);
+    stream_sum sum{0, 0};                   // of the column's first `have` tiles (first warp)
+    unsigned have = 0, column = 0, special = 0;
     bool missing = false;                   // one of them is not to be had
     for (uint32_t i = 0;; ++i) {
       const int st = (int)(i % N);
@@ -902,48 +1008,93 @@ __global__ void __launch_bounds__(kStreamThreads, 1)
       const unsigned long long t = s_tile[st];
       if (t == END) return;
       const unsigned k = s_k[st];
-      unsigned long long* a0 = agg + (t - k);
+      const int j = lane & 3;
+      unsigned long long* a0 = agg + (t - k) * kStreamWords + 2 * j;
       if (column != s_col[st]) {
         column = s_col[st];
-        groups = 0;
+        have = 0;
+        special = 0;
         missing = false;
-        mine = Op::template init<float>();
+        sum = stream_sum{0, 0};
       }
-      S part = mine;                        // with the last, incomplete round
-      constexpr int B = 6;
+      // lane l reads words 2 (l % 4) and the next of tile l / 4 of eight; B such
+      // loads in flight, and at most 2048 tiles before the digits are carried
+      constexpr unsigned B = kStreamLoads, STEP = 8 * kStreamGather, ROUND = 2048;
+      stream_sum more{0, 0};
 #pragma unroll 1
-      for (unsigned g = groups; g * 32u < k; g += B) {
-        unsigned long long w[B];
+      while (have < k) {
+        const unsigned end = k - have < ROUND ? k : have + ROUND;
+        unsigned long long x = 0, y = 0;
+        unsigned mine = 0, flags = 0;
+#pragma unroll 1
+        for (unsigned q0 = have + 8 * gw + (unsigned)(lane >> 2); q0 < end; q0 += STEP * B) {
+          ulonglong2 w[B];
+          unsigned long long all = 0;
 #pragma unroll
-        for (int b = 0; b < B; ++b) {
-          const unsigned q = (g + b) * 32u + (unsigned)lane;
-          w[b] = q < k ? stream_ld(a0 + q) : 0ull;
-        }
-#pragma unroll
-        for (int b = 0; b < B; ++b) {
-          const unsigned q = (g + b) * 32u + (unsigned)lane;
-          for (unsigned it = 0; w[b] == kStreamEmpty && it < kSpinMax; ++it) {
-            __nanosleep(20);
-            w[b] = stream_ld(a0 + q);
-          }
-          if (w[b] == kStreamEmpty) {       // give up, for every block that waits for it
-            atomicCAS(a0 + q, kStreamEmpty, kStreamFailed);
-            atomicAdd(&g_wait_timeouts, 1ull);
-            w[b] = kStreamFailed;
-          }
-          if (w[b] == kStreamFailed) missing = true;
-          if (q < k) {
-            part = Op::merge(mine, S{__uint_as_float((unsigned)w[b]), __uint_as_float((unsigned)(w[b] >> 32))});
-            if ((g + b) * 32u + 32u <= k) {
-              mine = part;
-              groups = g + b + 1;
+          for (unsigned b = 0; b < B; ++b) {
+            w[b] = ulonglong2{0, 0};
+            if (q0 + STEP * b < end) {
+              w[b] = stream_ld2(a0 + (size_t)(q0 + STEP * b) * kStreamWords);
+              ++mine;
             }
           }
+#pragma unroll
+          for (unsigned b = 0; b < B; ++b) all |= w[b].x | w[b].y;
+          if (all >> 62) {                  // some are not there yet
+#pragma unroll
+            for (unsigned b = 0; b < B; ++b) {
+              unsigned long long* p = a0 + (size_t)(q0 + STEP * b) * kStreamWords;
+              for (unsigned it = 0; (w[b].x == kStreamEmpty || w[b].y == kStreamEmpty) && it < kSpinMax; ++it) {
+                __nanosleep(20);
+                w[b] = stream_ld2(p);
+              }
+              if (w[b].x == kStreamEmpty || w[b].y == kStreamEmpty) {   // give up, for every block that waits for it
+                atomicCAS(p, kStreamEmpty, kStreamFailed);
+                atomicCAS(p + 1, kStreamEmpty, kStreamFailed);
+                atomicAdd(&g_wait_timeouts, 1ull);
+              }
+              if (stream_missing(w[b])) {
+                missing = true;
+                w[b] = ulonglong2{0, 0};
+              }
+            }
+          }
+#pragma unroll
+          for (unsigned b = 0; b < B; ++b) {
+            x += w[b].x;
+            y += w[b].y;
+            flags |= (unsigned)w[b].y;
+          }
         }
+        const unsigned long long bias = mine * kStreamBias;
+        const stream_sum a = stream_reduce(stream_sum{(long long)(x - bias), j < 3 ? (long long)(y - bias) : 0});
+        if (have + ROUND < k) stream_carry(more);
+        more.x += a.x;
+        more.y += a.y;
+        special |= __reduce_or_sync(0xffffffffu, j == 3 ? flags : 0u);
+        have = end;
       }
-      groups = __shfl_sync(0xffffffffu, groups, 0);
       missing = __any_sync(0xffffffffu, missing) != 0;
-      const S prefix = fold::warp_merge<Op, float>(part);
+      if (gw > 0) {
+        if (lane < 4) s_share[st][gw - 1][lane] = more;
+        if (lane == 0) s_flags[st][gw - 1] = special | (missing ? 8u : 0u);
+        __syncwarp();
+        if (lane == 0) tma::mbar_arrive(&shared_out[st]);
+        continue;
+      }
+      if (!wait(shared_out, i)) return;
+      unsigned found = special | (missing ? 8u : 0u);
+      sum.x += more.x;
+      sum.y += more.y;
+#pragma unroll
+      for (int o = 0; o < kStreamGather - 1; ++o) {
+        sum.x += s_share[st][o][j].x;
+        sum.y += s_share[st][o][j].y;
+        found |= s_flags[st][o];
+      }
+      stream_carry(sum);
+      missing = (found & 8u) != 0u;
+      const S prefix = stream_pair(sum, found & 7u);
       if (!wait(published, i)) return;
       if (lane < W) s_pre[st][lane] = Op::merge(prefix, s_ex[st][lane]);
       if (lane == 0) s_bad[st] = missing ? 1 : 0;
@@ -956,7 +1107,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1)
   if (lane != 0) return;
   uint32_t armed = 0, landed = 0;                                 // loads issued, and known to have arrived
   auto fetch = [&](int st) {
-    const unsigned long long t = atomicAdd(ticket, 1ull) + 1ull;  // the ticket starts at all ones
+    const unsigned long long t = atomicAdd(ticket, 1ull) - kStreamEmpty;   // what the ticket starts at, too
     s_tile[st] = t < sh.tiles ? t : END;
     if (t >= sh.tiles) {
       tma::mbar_arrive(&full[st]);

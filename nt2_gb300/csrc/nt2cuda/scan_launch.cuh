@@ -15,6 +15,16 @@ namespace scan {
 
 inline size_t align256(size_t b) { return (b + 255) / 256 * 256; }
 
+// Scratch of the look-back over `tiles` tiles: ticket and error word, flags,
+// aggregates, inclusive prefixes.
+constexpr size_t kScanHead = 256;
+inline size_t flag_bytes(size_t tiles) { return align256(tiles * sizeof(unsigned)); }
+template <class Op, class T> inline size_t side_bytes(size_t tiles) { return align256(tiles * carry_bytes<Op, T>()); }
+template <class Op, class T> inline size_t lookback_scratch(size_t tiles)
+{
+  return kScanHead + flag_bytes(tiles) + 2 * side_bytes<Op, T>(tiles);
+}
+
 // The streamed scan of long float columns (k_scan_stream).  cudaErrorNotSupported,
 // before anything is launched, when it does not apply.
 // At least a tile for each of 152 SMs (1.9 million floats 18.2 us before, 15.1),
@@ -48,14 +58,17 @@ cudaError_t inner_scan_stream(const float* x, float* y, size_t rows, size_t cols
       encode(&ymap, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, (void*)y, gdim, gstride, box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE,
              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return cudaErrorNotSupported;
-  // scratch: ticket | aggregates, all ones
+  // scratch: ticket | aggregates, all kStreamEmpty; never less than the look-back
+  // would take, so that a misaligned column of this shape can be captured after it
+  using K = scan_tiles<fold::op_sum<COMP>, float>;
   void* scratch = nullptr;
-  const size_t head = 256;
-  cudaError_t e = nt2cuda::stream_scratch(s, head + sh.tiles * 8, &scratch, 1);
+  const size_t head = kScanHead, sbytes = sh.tiles * kStreamWords * sizeof(unsigned long long);
+  const size_t other = lookback_scratch<fold::op_sum<COMP>, float>((rows + K::TILE - 1) / K::TILE * cols);
+  cudaError_t e = nt2cuda::stream_scratch(s, head + sbytes > other ? head + sbytes : other, &scratch, 1);
   if (e != cudaSuccess) return e;
   unsigned long long* ticket = (unsigned long long*)scratch;
   unsigned long long* agg = (unsigned long long*)((char*)scratch + head);
-  if ((e = cudaMemsetAsync(scratch, 0xff, head + sh.tiles * 8, s)) != cudaSuccess) return e;
+  if ((e = cudaMemsetAsync(scratch, 0x7f, head + sbytes, s)) != cudaSuccess) return e;
   auto k = k_scan_stream<COMP>;
   if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStreamSmem)) != cudaSuccess) return e;
   size_t grid = (size_t)sm_count();
@@ -87,10 +100,9 @@ cudaError_t inner_scan(const T* x, T* y, size_t rows, size_t cols, cudaStream_t 
   sh.tiles_per_col = (rows + TILE - 1) / TILE;
   sh.tiles = sh.tiles_per_col * cols;
   // scratch: ticket, error word, flags | aggregates | inclusive prefixes
-  const size_t head = 256, fbytes = align256(sh.tiles * sizeof(unsigned));
-  const size_t sbytes = align256(sh.tiles * carry_bytes<Op, T>());
+  const size_t head = kScanHead, fbytes = flag_bytes(sh.tiles), sbytes = side_bytes<Op, T>(sh.tiles);
   void* scratch = nullptr;
-  cudaError_t e = nt2cuda::stream_scratch(s, head + fbytes + 2 * sbytes, &scratch, 1);
+  cudaError_t e = nt2cuda::stream_scratch(s, lookback_scratch<Op, T>(sh.tiles), &scratch, 1);
   if (e != cudaSuccess) return e;
   char* b = (char*)scratch;
   unsigned long long* ticket = (unsigned long long*)b;
