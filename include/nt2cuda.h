@@ -441,6 +441,14 @@ nt2cuda_status nt2cuda_wait_timeouts(unsigned long long* count);
  * NT2CUDA_ERR_TIMEOUT when the kernel reported the timeout (the expected
  * result, after about a second), NT2CUDA_OK if it did not. */
 nt2cuda_status nt2cuda_selftest_wait_timeout(nt2cuda_stream stream);
+/* The same for the streamed scan, y = cumsum(x,1) of a 16-byte aligned rows x
+ * cols table long enough to be streamed.  kind 0: no block takes the first tile
+ * (12288 elements), which is left as it is; the rest of column 0 becomes NaN, the
+ * other columns are the normal result.  kind 1: every block gives up its own
+ * waits, and all of y becomes NaN.  Synchronous; returns NT2CUDA_ERR_TIMEOUT when
+ * the timeout was reported. */
+nt2cuda_status nt2cuda_selftest_stream_timeout(int kind, const float* x, size_t rows, size_t cols, float* y,
+                                               nt2cuda_stream stream);
 /* The same for the TMA column fold: out = sum(A,1) of a 16-byte aligned
  * rows x cols table (rows a multiple of 4 and above 65536, so every column is
  * split into several units) with the first tile of unit 0 armed but never

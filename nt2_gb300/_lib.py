@@ -94,6 +94,7 @@ _SIGS = {
     "nt2cuda_map2_f32": (c_int, [c_int, c_vp, c_vp, c_vp, c_size, c_int, c_vp]),
     "nt2cuda_map2_f64": (c_int, [c_int, c_vp, c_vp, c_vp, c_size, c_int, c_vp]),
     "nt2cuda_selftest_wait_timeout": (c_int, [c_vp]),
+    "nt2cuda_selftest_stream_timeout": (c_int, [c_int, c_vp, c_size, c_size, c_vp, c_vp]),
     "nt2cuda_selftest_fold_timeout": (c_int, [c_vp, c_size, c_size, c_vp, c_vp]),
     "nt2cuda_selftest_f64": (c_int, [c_int, C.POINTER(C.c_ulonglong), c_vp]),
     "nt2cuda_selftest_x2": (c_int, [c_int, C.POINTER(C.c_ulonglong), C.POINTER(C.c_uint32), c_vp]),

@@ -66,4 +66,13 @@ nt2cuda_status nt2cuda_selftest_wait_timeout(nt2cuda_stream s)
   return failed ? NT2CUDA_ERR_TIMEOUT : NT2CUDA_OK;
 }
 
+nt2cuda_status nt2cuda_selftest_stream_timeout(int kind, const float* x, size_t rows, size_t cols, float* y, nt2cuda_stream s)
+{
+  if (kind < 0 || kind > 1 || !x || !y || !rows || !cols) return NT2CUDA_ERR_ARG;
+  bool ran_out = false;
+  const nt2cuda_status st = from_cuda(scan::selftest_stream_timeout(kind, x, y, rows, cols, as_stream(s), &ran_out));
+  if (st != NT2CUDA_OK) return st;
+  return ran_out ? NT2CUDA_ERR_TIMEOUT : NT2CUDA_OK;
+}
+
 }  // extern "C"

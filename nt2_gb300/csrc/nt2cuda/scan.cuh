@@ -707,6 +707,11 @@ __global__ void __launch_bounds__(256, (scan_min_blocks<Op, T>::value)) k_scan_i
 // tile waits for anything but the arrival of tiles that running blocks hold,
 // and no block needs another to be resident.
 //
+// Every wait is bounded.  A gather that runs out marks the missing tile failed,
+// and every later tile of the column reads NaN.  A block whose own barrier wait
+// runs out stops: its roles leave their loops, its copies land, and its load/store
+// thread then writes NaN to the tiles it holds and to those it still draws.
+//
 // Roles, each a loop over the block's tiles with a barrier per stage between
 // them: load/store (one thread), fold (12 warps), publish (1), gather (5: the
 // tile's prefix), rescan (12).  (The 12 warps
@@ -717,7 +722,7 @@ __global__ void __launch_bounds__(256, (scan_min_blocks<Op, T>::value)) k_scan_i
 // The warps share the 152 or so tiles of a gather, so that its loads are in flight
 // at once: 2^26 floats 106 us with one or two warps, 102.6 with three of seven loads
 // a lane, 100.1 with five of four.)
-// 2^26 floats: 100 us, 79% of a copy of the same bytes (79 us); the two-pass tiles
+// 2^26 floats: 101 us, 78% of a copy of the same bytes (79 us); the two-pass tiles
 // with the look-back 151.  200000 x 200: 64.5 against 90.
 constexpr int kStreamWarps = 12, kStreamStages = 4;
 constexpr int kStreamRows = 32 * kStreamWarps;
@@ -732,6 +737,7 @@ constexpr unsigned long long kStreamBias = 1ull << 50;              // makes a p
 struct stream_shape {
   size_t rows, cols, tiles_per_col, tiles;
   uint32_t wait_rounds;            // of the block's own barriers
+  uint32_t polls;                  // of an aggregate that is not there yet
 };
 
 // Digit j (48 bits, weight 2^(48 j - 149)) of a finite float, with its sign.
@@ -800,7 +806,7 @@ __device__ __forceinline__ fold::acc<float> stream_pair(const stream_sum& r, uns
   using math::sub;
   const int lane = threadIdx.x & 31;
   if (special)
-    return fold::acc<float>{(special & 4u) || special == 3u ? nan_value<float>() : __int_as_float(special == 1u ? 0x7f800000 : (int)0xff800000u), 0.f};
+    return fold::acc<float>{special > 2u ? nan_value<float>() : __int_as_float(special == 1u ? 0x7f800000 : (int)0xff800000u), 0.f};
   const long long x = __shfl_sync(0xffffffffu, r.x, (lane >> 1) & 3), y = __shfl_sync(0xffffffffu, r.y, (lane >> 1) & 3);
   const long long d = lane < 7 ? ((lane & 1) ? y : x) : 0;           // lane l: digit l
   const unsigned nz = __ballot_sync(0xffffffffu, d != 0);
@@ -841,12 +847,15 @@ __device__ __forceinline__ void stream_st(unsigned long long* p, unsigned long l
   asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
-// Bounded wait that also ends when another warp of the block gave up.
-__device__ __forceinline__ bool stream_wait(uint64_t* bar, uint32_t phase, uint32_t rounds, const volatile int* abort)
+// Bounded wait that also ends when another warp of the block gave up.  Called by
+// whole warps (or lane 0 alone, `lanes` 1), whose lanes succeed or fail together:
+// one that left alone would be missed by the others' next shuffle.
+__device__ __forceinline__ bool stream_wait(uint64_t* bar, uint32_t phase, uint32_t rounds, const volatile int* abort,
+                                            unsigned lanes)
 {
   for (uint32_t i = 0; i < rounds; ++i) {
-    if (tma::mbar_try_wait(bar, phase)) return true;
-    if ((i & 15u) == 15u && *abort) return false;
+    if (__all_sync(lanes, tma::mbar_try_wait(bar, phase))) return true;
+    if ((i & 15u) == 15u && __any_sync(lanes, *abort)) return false;
   }
   return false;
 }
@@ -866,6 +875,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1)
   constexpr unsigned long long END = ~0ull;
   // one barrier of each kind per stage; tile i of the block is at stage i % N, phase (i / N) & 1
   __shared__ __align__(8) uint64_t full[N], folded[N], published[N], shared_out[N], prefixed[N], done[N];
+  __shared__ __align__(8) uint64_t gone;                          // the other warps have left their roles
   __shared__ unsigned long long s_tile[N];                        // the stage's tile
   __shared__ unsigned s_k[N], s_col[N];                           // its place in its column
   __shared__ S s_row[N][kStreamRows];                             // the rows' prefixes within their warp
@@ -885,12 +895,17 @@ __global__ void __launch_bounds__(kStreamThreads, 1)
       tma::mbar_init(&prefixed[q], 1);
       tma::mbar_init(&done[q], W);
     }
+    tma::mbar_init(&gone, 2 * W + 1 + kStreamGather);
     s_abort = 0;
     tma::fence_barrier_init();
   }
   __syncthreads();
-  auto wait = [&](uint64_t* bars, uint32_t i) {
-    if (stream_wait(&bars[i % N], (i / N) & 1u, sh.wait_rounds, &s_abort)) return true;
+  auto draw = [&] {                                               // the next tile
+    const unsigned long long t = atomicAdd(ticket, 1ull) - kStreamEmpty;   // what the ticket starts at, too
+    return t < sh.tiles ? t : END;
+  };
+  auto wait = [&](uint64_t* bars, uint32_t i, unsigned lanes = 0xffffffffu) {
+    if (stream_wait(&bars[i % N], (i / N) & 1u, sh.wait_rounds, &s_abort, lanes)) return true;
     if (lane == 0 && atomicExch(&s_abort, 1) == 0) atomicAdd(&g_wait_timeouts, 1ull);
     return false;
   };
@@ -899,217 +914,228 @@ __global__ void __launch_bounds__(kStreamThreads, 1)
     return reinterpret_cast<float4*>(stage0 + (size_t)st * TBYTES + (size_t)row * 128 + (size_t)((c ^ (row & 7)) * 16));
   };
 
-  if (warp < W) {
-    // ---------------------------------------------------------------- fold
-    const int row = (int)threadIdx.x;
-    for (uint32_t i = 0;; ++i) {
-      const int st = (int)(i % N);
-      if (!wait(full, i) || s_tile[st] == END) return;
-      S c = Op::template init<float>();
+  // the roles but the last; each returns after the block's last tile, or when a wait of the block ran out
+  auto roles = [&] {
+    if (warp < W) {
+      // ---------------------------------------------------------------- fold
+      const int row = (int)threadIdx.x;
+      for (uint32_t i = 0;; ++i) {
+        const int st = (int)(i % N);
+        if (!wait(full, i) || s_tile[st] == END) return;
+        S c = Op::template init<float>();
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const float4 v = *chunk(st, row, q);
-        Op::add(c, v.x);
-        Op::add(c, v.y);
-        Op::add(c, v.z);
-        Op::add(c, v.w);
-      }
+        for (int q = 0; q < 8; ++q) {
+          const float4 v = *chunk(st, row, q);
+          Op::add(c, v.x);
+          Op::add(c, v.y);
+          Op::add(c, v.z);
+          Op::add(c, v.w);
+        }
 #pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const S o = Op::shfl_from(c, lane >= d ? lane - d : 0);
-        if (lane >= d) c = Op::merge(o, c);
-      }
-      S ex = Op::shfl_from(c, lane > 0 ? lane - 1 : 0);
-      if (lane == 0) ex = Op::template init<float>();
-      s_row[st][row] = ex;
-      if (lane == 31) s_tot[st][warp] = c;
-      __syncwarp();
-      if (lane == 31) tma::mbar_arrive(&folded[st]);
-    }
-  }
-
-  if (warp < 2 * W) {
-    // -------------------------------------------------------------- rescan
-    const int w = warp - W, row = (int)threadIdx.x - 32 * W;
-    const size_t rows32 = sh.rows / 32;
-    const int rest = (int)(sh.rows % 32);
-    const float nan = nan_value<float>();
-    for (uint32_t i = 0;; ++i) {
-      const int st = (int)(i % N);
-      if (!wait(full, i) || s_tile[st] == END) return;
-      if (!wait(prefixed, i)) return;
-      S acc = Op::merge(s_pre[st][w], s_row[st][row]);
-      const bool bad = s_bad[st] != 0;
-      const size_t r = (size_t)s_k[st] * kStreamRows + (size_t)row;
-      const size_t base = (size_t)s_col[st] * sh.rows + rows32 * 32;
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        float4 v = *chunk(st, row, q);
-        Op::add(acc, v.x);
-        v.x = bad ? nan : Op::finish(acc, 0);
-        Op::add(acc, v.y);
-        v.y = bad ? nan : Op::finish(acc, 0);
-        Op::add(acc, v.z);
-        v.z = bad ? nan : Op::finish(acc, 0);
-        Op::add(acc, v.w);
-        v.w = bad ? nan : Op::finish(acc, 0);
-        *chunk(st, row, q) = v;
-      }
-      tma::fence_proxy_async();
-      __syncwarp();
-      if (lane == 0) tma::mbar_arrive(&done[st]);
-      if (rest && r + 1 == rows32) {              // the column's last rows % 32 elements, after its last whole row
-        float v[31];
-#pragma unroll
-        for (int e = 0; e < 31; ++e) v[e] = e < rest ? x[base + e] : 0.f;
-#pragma unroll
-        for (int e = 0; e < 31; ++e)
-          if (e < rest) {
-            Op::add(acc, v[e]);
-            y[base + e] = bad ? nan : Op::finish(acc, 0);
-          }
+        for (int d = 1; d < 32; d <<= 1) {
+          const S o = Op::shfl_from(c, lane >= d ? lane - d : 0);
+          if (lane >= d) c = Op::merge(o, c);
+        }
+        S ex = Op::shfl_from(c, lane > 0 ? lane - 1 : 0);
+        if (lane == 0) ex = Op::template init<float>();
+        s_row[st][row] = ex;
+        if (lane == 31) s_tot[st][warp] = c;
+        __syncwarp();
+        if (lane == 31) tma::mbar_arrive(&folded[st]);
       }
     }
-  }
 
-  if (warp == 2 * W) {
-    // ------------------------------------------------------------- publish
-    for (uint32_t i = 0;; ++i) {
-      const int st = (int)(i % N);
-      if (!wait(full, i)) return;
-      const unsigned long long t = s_tile[st];
-      if (t == END || !wait(folded, i)) return;
-      S c = lane < W ? s_tot[st][lane] : Op::template init<float>();
+    if (warp < 2 * W) {
+      // -------------------------------------------------------------- rescan
+      const int w = warp - W, row = (int)threadIdx.x - 32 * W;
+      const size_t rows32 = sh.rows / 32;
+      const int rest = (int)(sh.rows % 32);
+      const float nan = nan_value<float>();
+      for (uint32_t i = 0;; ++i) {
+        const int st = (int)(i % N);
+        if (!wait(full, i) || s_tile[st] == END) return;
+        if (!wait(prefixed, i)) return;
+        S acc = Op::merge(s_pre[st][w], s_row[st][row]);
+        const bool bad = s_bad[st] != 0;
+        const size_t r = (size_t)s_k[st] * kStreamRows + (size_t)row;
+        const size_t base = (size_t)s_col[st] * sh.rows + rows32 * 32;
 #pragma unroll
-      for (int d = 1; d < 16; d <<= 1) {
-        const S o = Op::shfl_from(c, lane >= d ? lane - d : 0);
-        if (lane >= d) c = Op::merge(o, c);
-      }
-      const S tile = Op::shfl_from(c, W - 1);
-      if (lane < kStreamWords) stream_st(agg + t * kStreamWords + lane, stream_word(tile, lane));
-      S ex = Op::shfl_from(c, lane > 0 ? lane - 1 : 0);
-      if (lane == 0) ex = Op::template init<float>();
-      if (lane < W) s_ex[st][lane] = ex;
-      __syncwarp();
-      if (lane == 0) tma::mbar_arrive(&published[st]);
-    }
-  }
-
-  if (warp <= 2 * W + kStreamGather) {
-    // -------------------------------------------------------------- gather
-    // (each of the warps a share of the tiles; the first one puts the shares together)
-    const int gw = warp - (2 * W + 1);
-    stream_sum sum{0, 0};                   // of the column's first `have` tiles (first warp)
-    unsigned have = 0, column = 0, special = 0;
-    bool missing = false;                   // one of them is not to be had
-    for (uint32_t i = 0;; ++i) {
-      const int st = (int)(i % N);
-      if (!wait(full, i)) return;
-      const unsigned long long t = s_tile[st];
-      if (t == END) return;
-      const unsigned k = s_k[st];
-      const int j = lane & 3;
-      unsigned long long* a0 = agg + (t - k) * kStreamWords + 2 * j;
-      if (column != s_col[st]) {
-        column = s_col[st];
-        have = 0;
-        special = 0;
-        missing = false;
-        sum = stream_sum{0, 0};
-      }
-      // lane l reads words 2 (l % 4) and the next of tile l / 4 of eight; B such
-      // loads in flight, and at most 2048 tiles before the digits are carried
-      constexpr unsigned B = kStreamLoads, STEP = 8 * kStreamGather, ROUND = 2048;
-      stream_sum more{0, 0};
-#pragma unroll 1
-      while (have < k) {
-        const unsigned end = k - have < ROUND ? k : have + ROUND;
-        unsigned long long x = 0, y = 0;
-        unsigned mine = 0, flags = 0;
-#pragma unroll 1
-        for (unsigned q0 = have + 8 * gw + (unsigned)(lane >> 2); q0 < end; q0 += STEP * B) {
-          ulonglong2 w[B];
-          unsigned long long all = 0;
+        for (int q = 0; q < 8; ++q) {
+          float4 v = *chunk(st, row, q);
+          Op::add(acc, v.x);
+          v.x = bad ? nan : Op::finish(acc, 0);
+          Op::add(acc, v.y);
+          v.y = bad ? nan : Op::finish(acc, 0);
+          Op::add(acc, v.z);
+          v.z = bad ? nan : Op::finish(acc, 0);
+          Op::add(acc, v.w);
+          v.w = bad ? nan : Op::finish(acc, 0);
+          *chunk(st, row, q) = v;
+        }
+        tma::fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) tma::mbar_arrive(&done[st]);
+        if (rest && r + 1 == rows32) {              // the column's last rows % 32 elements, after its last whole row
+          float v[31];
 #pragma unroll
-          for (unsigned b = 0; b < B; ++b) {
-            w[b] = ulonglong2{0, 0};
-            if (q0 + STEP * b < end) {
-              w[b] = stream_ld2(a0 + (size_t)(q0 + STEP * b) * kStreamWords);
-              ++mine;
+          for (int e = 0; e < 31; ++e) v[e] = e < rest ? x[base + e] : 0.f;
+#pragma unroll
+          for (int e = 0; e < 31; ++e)
+            if (e < rest) {
+              Op::add(acc, v[e]);
+              y[base + e] = bad ? nan : Op::finish(acc, 0);
             }
-          }
+        }
+      }
+    }
+
+    if (warp == 2 * W) {
+      // ------------------------------------------------------------- publish
+      for (uint32_t i = 0;; ++i) {
+        const int st = (int)(i % N);
+        if (!wait(full, i)) return;
+        const unsigned long long t = s_tile[st];
+        if (t == END || !wait(folded, i)) return;
+        S c = lane < W ? s_tot[st][lane] : Op::template init<float>();
 #pragma unroll
-          for (unsigned b = 0; b < B; ++b) all |= w[b].x | w[b].y;
-          if (all >> 62) {                  // some are not there yet
+        for (int d = 1; d < 16; d <<= 1) {
+          const S o = Op::shfl_from(c, lane >= d ? lane - d : 0);
+          if (lane >= d) c = Op::merge(o, c);
+        }
+        const S tile = Op::shfl_from(c, W - 1);
+        if (lane < kStreamWords) stream_st(agg + t * kStreamWords + lane, stream_word(tile, lane));
+        S ex = Op::shfl_from(c, lane > 0 ? lane - 1 : 0);
+        if (lane == 0) ex = Op::template init<float>();
+        if (lane < W) s_ex[st][lane] = ex;
+        __syncwarp();
+        if (lane == 0) tma::mbar_arrive(&published[st]);
+      }
+    }
+
+    if (warp <= 2 * W + kStreamGather) {
+      // -------------------------------------------------------------- gather
+      // (each of the warps a share of the tiles; the first one puts the shares together)
+      const int gw = warp - (2 * W + 1);
+      stream_sum sum{0, 0};                   // of the column's first `have` tiles (first warp)
+      unsigned have = 0, column = 0, special = 0;
+      bool missing = false;                   // one of them is not to be had
+      for (uint32_t i = 0;; ++i) {
+        const int st = (int)(i % N);
+        if (!wait(full, i)) return;
+        const unsigned long long t = s_tile[st];
+        if (t == END) return;
+        const unsigned k = s_k[st];
+        const int j = lane & 3;
+        unsigned long long* a0 = agg + (t - k) * kStreamWords + 2 * j;
+        if (column != s_col[st]) {
+          column = s_col[st];
+          have = 0;
+          special = 0;
+          missing = false;
+          sum = stream_sum{0, 0};
+        }
+        // lane l reads words 2 (l % 4) and the next of tile l / 4 of eight; B such
+        // loads in flight, and at most 2048 tiles before the digits are carried
+        constexpr unsigned B = kStreamLoads, STEP = 8 * kStreamGather, ROUND = 2048;
+        stream_sum more{0, 0};
+#pragma unroll 1
+        while (have < k) {
+          const unsigned end = k - have < ROUND ? k : have + ROUND;
+          unsigned long long x = 0, y = 0;
+          unsigned mine = 0, flags = 0;
+#pragma unroll 1
+          for (unsigned q0 = have + 8 * gw + (unsigned)(lane >> 2); q0 < end; q0 += STEP * B) {
+            ulonglong2 w[B];
+            unsigned long long all = 0;
 #pragma unroll
             for (unsigned b = 0; b < B; ++b) {
-              unsigned long long* p = a0 + (size_t)(q0 + STEP * b) * kStreamWords;
-              for (unsigned it = 0; (w[b].x == kStreamEmpty || w[b].y == kStreamEmpty) && it < kSpinMax; ++it) {
-                __nanosleep(20);
-                w[b] = stream_ld2(p);
-              }
-              if (w[b].x == kStreamEmpty || w[b].y == kStreamEmpty) {   // give up, for every block that waits for it
-                atomicCAS(p, kStreamEmpty, kStreamFailed);
-                atomicCAS(p + 1, kStreamEmpty, kStreamFailed);
-                atomicAdd(&g_wait_timeouts, 1ull);
-              }
-              if (stream_missing(w[b])) {
-                missing = true;
-                w[b] = ulonglong2{0, 0};
+              w[b] = ulonglong2{0, 0};
+              if (q0 + STEP * b < end) {
+                w[b] = stream_ld2(a0 + (size_t)(q0 + STEP * b) * kStreamWords);
+                ++mine;
               }
             }
-          }
 #pragma unroll
-          for (unsigned b = 0; b < B; ++b) {
-            x += w[b].x;
-            y += w[b].y;
-            flags |= (unsigned)w[b].y;
+            for (unsigned b = 0; b < B; ++b) all |= w[b].x | w[b].y;
+            if (all >> 62) {                  // some are not there yet
+#pragma unroll
+              for (unsigned b = 0; b < B; ++b) {
+                unsigned long long* p = a0 + (size_t)(q0 + STEP * b) * kStreamWords;
+                const unsigned polls = missing ? 0u : sh.polls;   // one wait of a column may run out, not one for each tile
+                for (unsigned it = 0; (w[b].x == kStreamEmpty || w[b].y == kStreamEmpty) && it < polls; ++it) {
+                  __nanosleep(20);
+                  w[b] = stream_ld2(p);
+                }
+                if (w[b].x == kStreamEmpty || w[b].y == kStreamEmpty) {   // give up, for every block that waits for it
+                  atomicCAS(p, kStreamEmpty, kStreamFailed);
+                  atomicCAS(p + 1, kStreamEmpty, kStreamFailed);
+                  atomicAdd(&g_wait_timeouts, 1ull);
+                }
+                if (stream_missing(w[b])) {
+                  missing = true;
+                  w[b] = ulonglong2{0, 0};
+                }
+              }
+            }
+#pragma unroll
+            for (unsigned b = 0; b < B; ++b) {
+              x += w[b].x;
+              y += w[b].y;
+              flags |= (unsigned)w[b].y;
+            }
           }
+          const unsigned long long bias = mine * kStreamBias;
+          const stream_sum a = stream_reduce(stream_sum{(long long)(x - bias), j < 3 ? (long long)(y - bias) : 0});
+          if (have + ROUND < k) stream_carry(more);
+          more.x += a.x;
+          more.y += a.y;
+          special |= __reduce_or_sync(0xffffffffu, j == 3 ? flags : 0u);
+          have = end;
         }
-        const unsigned long long bias = mine * kStreamBias;
-        const stream_sum a = stream_reduce(stream_sum{(long long)(x - bias), j < 3 ? (long long)(y - bias) : 0});
-        if (have + ROUND < k) stream_carry(more);
-        more.x += a.x;
-        more.y += a.y;
-        special |= __reduce_or_sync(0xffffffffu, j == 3 ? flags : 0u);
-        have = end;
-      }
-      missing = __any_sync(0xffffffffu, missing) != 0;
-      if (gw > 0) {
-        if (lane < 4) s_share[st][gw - 1][lane] = more;
-        if (lane == 0) s_flags[st][gw - 1] = special | (missing ? 8u : 0u);
-        __syncwarp();
-        if (lane == 0) tma::mbar_arrive(&shared_out[st]);
-        continue;
-      }
-      if (!wait(shared_out, i)) return;
-      unsigned found = special | (missing ? 8u : 0u);
-      sum.x += more.x;
-      sum.y += more.y;
+        missing = __any_sync(0xffffffffu, missing) != 0;
+        if (gw > 0) {
+          if (lane < 4) s_share[st][gw - 1][lane] = more;
+          if (lane == 0) s_flags[st][gw - 1] = special | (missing ? 8u : 0u);
+          __syncwarp();
+          if (lane == 0) tma::mbar_arrive(&shared_out[st]);
+          continue;
+        }
+        if (!wait(shared_out, i)) return;
+        unsigned found = special | (missing ? 8u : 0u);
+        sum.x += more.x;
+        sum.y += more.y;
 #pragma unroll
-      for (int o = 0; o < kStreamGather - 1; ++o) {
-        sum.x += s_share[st][o][j].x;
-        sum.y += s_share[st][o][j].y;
-        found |= s_flags[st][o];
+        for (int o = 0; o < kStreamGather - 1; ++o) {
+          sum.x += s_share[st][o][j].x;
+          sum.y += s_share[st][o][j].y;
+          found |= s_flags[st][o];
+        }
+        stream_carry(sum);
+        missing = (found & 8u) != 0u;
+        const S prefix = stream_pair(sum, found & 7u);
+        if (!wait(published, i)) return;
+        if (lane < W) s_pre[st][lane] = Op::merge(prefix, s_ex[st][lane]);
+        if (lane == 0) s_bad[st] = missing ? 1 : 0;
+        __syncwarp();
+        if (lane == 0) tma::mbar_arrive(&prefixed[st]);
       }
-      stream_carry(sum);
-      missing = (found & 8u) != 0u;
-      const S prefix = stream_pair(sum, found & 7u);
-      if (!wait(published, i)) return;
-      if (lane < W) s_pre[st][lane] = Op::merge(prefix, s_ex[st][lane]);
-      if (lane == 0) s_bad[st] = missing ? 1 : 0;
-      __syncwarp();
-      if (lane == 0) tma::mbar_arrive(&prefixed[st]);
     }
+  };
+  if (warp < 2 * W + 1 + kStreamGather) {
+    roles();
+    __syncwarp();
+    if (lane == 0) tma::mbar_arrive(&gone);
+    return;
   }
 
   // ------------------------------------------------------ loads and stores
   if (lane != 0) return;
+  bool stopped = false;
   uint32_t armed = 0, landed = 0;                                 // loads issued, and known to have arrived
   auto fetch = [&](int st) {
-    const unsigned long long t = atomicAdd(ticket, 1ull) - kStreamEmpty;   // what the ticket starts at, too
-    s_tile[st] = t < sh.tiles ? t : END;
-    if (t >= sh.tiles) {
+    const unsigned long long t = draw();
+    s_tile[st] = t;
+    if (t == END) {
       tma::mbar_arrive(&full[st]);
       return;
     }
@@ -1133,7 +1159,10 @@ __global__ void __launch_bounds__(kStreamThreads, 1)
   for (uint32_t i = 0;; ++i) {
     const int st = (int)(i % N);
     if (s_tile[st] == END) break;
-    if (!wait(done, i)) break;
+    if (!wait(done, i, 1u)) {
+      stopped = true;
+      break;
+    }
     ++landed;
     const int r0 = (int)s_k[st] * kStreamRows, col = (int)s_col[st];
     const unsigned char* buf = stage0 + (size_t)st * TBYTES;
@@ -1145,9 +1174,21 @@ __global__ void __launch_bounds__(kStreamThreads, 1)
     fetch(st);
   }
   // copies still in flight land in this block's shared memory (a wait gave up): wait for them, bounded
-  for (; landed < armed; ++landed)
-    tma::mbar_wait(&full[landed % N], (landed / N) & 1u, sh.wait_rounds);
+  for (; landed < armed; ++landed) tma::mbar_wait(&full[landed % N], (landed / N) & 1u);
   tma::bulk_wait<0>();
+  if (!stopped) return;
+  // A wait ran out: the tiles of the stages, which no store has taken, and all
+  // that are still to be handed out to this block read NaN.
+  tma::mbar_wait(&gone, 0);
+  auto give_up = [&](unsigned long long t) {
+    const size_t col = (size_t)(t / sh.tiles_per_col), k = (size_t)(t % sh.tiles_per_col);
+    const size_t r1 = k + 1 == sh.tiles_per_col ? sh.rows : (k + 1) * kStreamTile;
+    for (size_t r = k * kStreamTile; r < r1; ++r) y[col * sh.rows + r] = nan_value<float>();
+    for (int j = 0; j < kStreamWords; ++j) atomicCAS(agg + t * kStreamWords + j, kStreamEmpty, kStreamFailed);
+  };
+  for (int st = 0; st < N; ++st)
+    if (s_tile[st] != END) give_up(s_tile[st]);
+  for (unsigned long long t = draw(); t != END; t = draw()) give_up(t);
 }
 
 // Columns of at most one 32 KB tile (8 warps x 32 lanes x 8 consecutive

@@ -33,8 +33,11 @@ template <class Op, class T> inline size_t lookback_scratch(size_t tiles)
 constexpr size_t kStreamTiles = 152;
 template <class Op, class T> struct streamed { static constexpr bool value = false; };
 template <bool COMP> struct streamed<fold::op_sum<COMP>, float> { static constexpr bool value = true; static constexpr bool comp = COMP; };
+// first, wait_rounds and polls are for the timeout self-test: the tile handed out
+// first, and the bounds of the waits.
 template <bool COMP>
-cudaError_t inner_scan_stream(const float* x, float* y, size_t rows, size_t cols, cudaStream_t s)
+cudaError_t inner_scan_stream(const float* x, float* y, size_t rows, size_t cols, cudaStream_t s, unsigned first = 0,
+                              uint32_t wait_rounds = tma::kMaxRounds, uint32_t polls = kSpinMax)
 {
   if (rows < kStreamTile || rows / 32 >= ((size_t)1 << 31) || cols >= ((size_t)1 << 31) || (cols > 1 && rows % 4) ||
       (((uintptr_t)x | (uintptr_t)y) & 15u))
@@ -44,7 +47,8 @@ cudaError_t inner_scan_stream(const float* x, float* y, size_t rows, size_t cols
   sh.cols = cols;
   sh.tiles_per_col = (rows / 32 + kStreamRows - 1) / kStreamRows;
   sh.tiles = sh.tiles_per_col * cols;
-  sh.wait_rounds = tma::kMaxRounds;
+  sh.wait_rounds = wait_rounds;
+  sh.polls = polls;
   if (sh.tiles < kStreamTiles || sh.tiles_per_col * kStreamTile > rows + rows / 8) return cudaErrorNotSupported;
   PFN_cuTensorMapEncodeTiled_v12000 encode = tma::tensor_map_encoder();
   if (!encode) return cudaErrorNotSupported;
@@ -69,6 +73,7 @@ cudaError_t inner_scan_stream(const float* x, float* y, size_t rows, size_t cols
   unsigned long long* ticket = (unsigned long long*)scratch;
   unsigned long long* agg = (unsigned long long*)((char*)scratch + head);
   if ((e = cudaMemsetAsync(scratch, 0x7f, head + sbytes, s)) != cudaSuccess) return e;
+  if (first && (e = cudaMemsetAsync(scratch, 0x7f + (int)first, 1, s)) != cudaSuccess) return e;
   auto k = k_scan_stream<COMP>;
   if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStreamSmem)) != cudaSuccess) return e;
   size_t grid = (size_t)sm_count();
@@ -169,6 +174,23 @@ inline cudaError_t selftest_wait_timeout(cudaStream_t s, unsigned* failed)
   }
   if (buf) cudaFree(buf);
   if (scratch) cudaFree(scratch);
+  return e;
+}
+
+// The same for the streamed scan of x (which must be one it takes) into y.  kind 0:
+// the tile at 0 is handed out to no block, so the gathers of the others run out;
+// kind 1: no block waits for its own barriers at all.
+inline cudaError_t selftest_stream_timeout(int kind, const float* x, float* y, size_t rows, size_t cols, cudaStream_t s,
+                                           bool* ran_out)
+{
+  unsigned long long before = 0, after = 0;
+  cudaError_t e = read_scan_wait_timeouts(&before);
+  if (e == cudaSuccess)
+    e = kind == 0 ? inner_scan_stream<true>(x, y, rows, cols, s, 1, tma::kMaxRounds, 1u << 10)
+                  : inner_scan_stream<true>(x, y, rows, cols, s, 0, 0);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  if (e == cudaSuccess) e = read_scan_wait_timeouts(&after);
+  *ran_out = after > before;
   return e;
 }
 
