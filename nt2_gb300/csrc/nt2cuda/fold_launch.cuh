@@ -34,11 +34,11 @@ template <class E> bool expr_aligned(const E& e)
 // elements, so that a few long columns fill the chip too (3333333 x 1 floats:
 // 44 us with segments of 16384, 10.5 with 2432 of them), but never below eight
 // loads a lane, and at most kInnerSplits to a column, as one warp merges them.
-// The cut depends on the table's shape alone: results are reproducible.
+// The cut depends on the table's shape alone (and on whether the call is captured,
+// see captured_cut): results are reproducible.
 // (var/stdev of doubles: 16 a SM in either case, what their 128 registers leave
 // room for; 70000 x 111: 46.9 us with 8, 40.7 with 16, 41.6 with 24.)
 constexpr size_t kInnerUnits = 3648, kInnerUnitsScalar = 2432, kInnerSplits = 2432;
-constexpr size_t kInnerWhole = 4096;     // 16-byte groups of the longest column folded whole under capture
 template <class Op, class T> inline size_t inner_seg(size_t rows, size_t cols, bool vec)
 {
   const size_t lanes = vec ? 32 * (16 / sizeof(T)) : 32;
@@ -90,6 +90,16 @@ template <bool W1, bool SD, class E> struct outer_unroll<op_moments<W1, SD>, flo
 constexpr int kScalarUnroll = 16;
 constexpr size_t kOuterUnits = 608;
 
+// Segments of inner_fold under capture (captured_cut): 128 loads of 16 bytes a lane,
+// or 16 bulk-copy tiles where a column of double var/stdev would otherwise be staged.
+template <class Op, class T, class E> inline size_t inner_wide(size_t rows, bool vec)
+{
+  constexpr size_t VV = 16 / sizeof(T), seg = 32 * VV * 128;
+  if (warp_framed<Op, T>::value && tma_terms<E>::n > 0 && vec && rows >= ((size_t)1 << 16))
+    return (size_t)inner_tile<T>() * 16;
+  return seg;
+}
+
 template <class Op, class T> cudaError_t fold_empty(out_of<Op, T>* out, size_t count, cudaStream_t s)
 {
   void* args[] = {&out, &count};
@@ -130,19 +140,15 @@ cudaError_t inner_fold(const E& e, size_t rows, size_t cols, out_of<Op, T>* out,
   sh.cols = cols;
   sh.seg = inner_seg<Op, T>(rows, cols, vec);
   sh.splits = (rows + sh.seg - 1) / sh.seg;
-  // a stream captured before its scratch was allocated: columns of one warp each
-  if (sh.splits > 1 && rows <= kInnerWhole * VV && fold_scratch_barred(s, cols, cols * sh.splits, sizeof(S))) {
-    sh.seg = round_up(rows, 32 * VV);
-    sh.splits = 1;
+  const size_t wide_seg = inner_wide<Op, T, E>(rows, vec), wide = (rows + wide_seg - 1) / wide_seg;
+  if (captured_cut(sh.splits, wide, s) != sh.splits) {
+    sh.seg = wide_seg;
+    sh.splits = wide;
   }
-  S* partials = nullptr;
+  void* partials = nullptr;
   unsigned* counters = nullptr;
-  if (sh.splits > 1) {
-    void* p = nullptr;
-    cudaError_t st = fold_scratch(s, cols, cols * sh.splits, sizeof(S), &counters, &p);
-    if (st != cudaSuccess) return st;
-    partials = (S*)p;
-  }
+  const cudaError_t st = fold_scratch(s, cols, sh.splits, wide, sizeof(S), &counters, &partials);
+  if (st != cudaSuccess) return st;
   const size_t units = cols * sh.splits;
   E ec = e;
   out_of<Op, T>* o = out;
@@ -181,22 +187,22 @@ cudaError_t outer_fold(const E& e, size_t rows, size_t cols, out_of<Op, T>* out,
   sh.cols = cols;
   sh.strips = (rows + STRIP - 1) / STRIP;
   // as many chunks as keep the blocks within 608, four a SM: one wave, every
-  // block at once (8192 x 4096 floats in 640 blocks takes 29.8 us); the split
-  // depends only on the shape, so results stay reproducible
-  {
-    const size_t want = sh.strips < kOuterUnits ? kOuterUnits / sh.strips : 1;
-    const size_t cchunk = round_up((cols + want - 1) / want, 8);
-    sh.cchunk = cchunk < 64 ? 64 : cchunk;
-  }
+  // block at once (8192 x 4096 floats in 640 blocks takes 29.8 us); under capture
+  // (captured_cut) whole 64 columns in about 512 blocks.  The split depends only on
+  // the shape, so results stay reproducible.
+  const size_t want = sh.strips < kOuterUnits ? kOuterUnits / sh.strips : 1, wide_want = (512 + sh.strips - 1) / sh.strips;
+  const size_t chunk = round_up((cols + want - 1) / want, 8), wide_chunk = round_up((cols + wide_want - 1) / wide_want, 64);
+  sh.cchunk = chunk < 64 ? 64 : chunk;
   sh.splits = (cols + sh.cchunk - 1) / sh.cchunk;
-  S* partials = nullptr;
-  unsigned* counters = nullptr;
-  if (sh.splits > 1) {
-    void* p = nullptr;
-    cudaError_t st = fold_scratch(s, sh.strips, sh.strips * sh.splits * STRIP, sizeof(S), &counters, &p);
-    if (st != cudaSuccess) return st;
-    partials = (S*)p;
+  const size_t wide = (cols + wide_chunk - 1) / wide_chunk;
+  if (captured_cut(sh.splits, wide, s) != sh.splits) {
+    sh.cchunk = wide_chunk;
+    sh.splits = wide;
   }
+  void* partials = nullptr;
+  unsigned* counters = nullptr;
+  const cudaError_t st = fold_scratch(s, sh.strips, sh.splits, wide, sizeof(S), &counters, &partials, STRIP);
+  if (st != cudaSuccess) return st;
   const size_t units = sh.strips * sh.splits;
   E ec = e;
   out_of<Op, T>* o = out;

@@ -433,6 +433,18 @@ __global__ void __launch_bounds__(256) k_outer_tma(const __grid_constant__ CUten
 // ------------------------------------------------------------- launchers
 using tma::tensor_map_encoder;
 
+// Segments of a column (of a row, the outer fold) that a captured call takes: as
+// `wide` cuts it, if that is less than `splits`.  A graph keeps the addresses of its
+// stream's partials and counters, and shares them with the graphs and calls of that
+// stream that it may later overlap with; so a column of up to 4096 16-byte groups
+// needs none, and longer ones no more than 128 of them a lane took, so that what a
+// stream's scratch was large enough for stays so.  Outside capture the scratch is
+// made large enough for either cut.
+inline size_t captured_cut(size_t splits, size_t wide, cudaStream_t s)
+{
+  return splits > wide && capturing(s) ? wide : splits;
+}
+
 template <class K> inline cudaError_t set_smem(K kernel, int bytes)
 {
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
@@ -451,25 +463,20 @@ cudaError_t inner_fold_tma(const T* x, const T* y, size_t rows, size_t cols, out
   sh.cols = cols;
   sh.seg = inner_tma_seg<T>(rows, cols, y ? 2 : 1);
   sh.splits = (rows + sh.seg - 1) / sh.seg;
-  // a stream captured before its scratch was allocated: columns of one unit each
-  if (sh.splits > 1 && rows <= (size_t)TILE * 16 && fold_scratch_barred(s, cols, cols * sh.splits, sizeof(S))) {
-    sh.seg = rows;
-    sh.splits = 1;
+  const size_t wide_seg = (size_t)TILE * 16, wide = (rows + wide_seg - 1) / wide_seg;
+  if (captured_cut(sh.splits, wide, s) != sh.splits) {
+    sh.seg = wide_seg;
+    sh.splits = wide;
   }
   sh.units = cols * sh.splits;
   sh.fail_unit = fail_unit;
   sh.wait_rounds = wait_rounds;
   if (sh.units == 0) return cudaSuccess;
-  S* partials = nullptr;
+  void* partials = nullptr;
   unsigned* counters = nullptr;
-  if (sh.splits > 1) {
-    void* p = nullptr;
-    cudaError_t e = fold_scratch(s, cols, sh.units, sizeof(S), &counters, &p);
-    if (e != cudaSuccess) return e;
-    partials = (S*)p;
-  }
+  cudaError_t e = fold_scratch(s, cols, sh.splits, wide, sizeof(S), &counters, &partials);
+  if (e != cudaSuccess) return e;
   size_t grid;
-  cudaError_t e;
   if (y) {
     constexpr int ST = 3;
     auto k = k_inner_tma<Op, T, 2, ST>;
@@ -528,18 +535,14 @@ cudaError_t outer_fold_tma(const T* A, size_t rows, size_t cols, out_of<Op, T>* 
   sh.splits = (cols + sh.cchunk - 1) / sh.cchunk;
   sh.units = sh.strips * sh.splits;
   sh.wait_rounds = tma::kMaxRounds;
-  S* partials = nullptr;
+  void* partials = nullptr;
   unsigned* counters = nullptr;
-  if (sh.splits > 1) {
-    void* p = nullptr;
-    cudaError_t e = fold_scratch(s, sh.strips, sh.units * BR, sizeof(S), &counters, &p);
-    if (e != cudaSuccess) return e;
-    partials = (S*)p;
-  }
+  cudaError_t e = fold_scratch(s, sh.strips, sh.splits, sh.splits, sizeof(S), &counters, &partials, BR);
+  if (e != cudaSuccess) return e;
   constexpr int ST = 4;
   auto k = k_outer_tma<Op, T, ST>;
   const int smem = ST * kTmaTileBytes;
-  cudaError_t e = set_smem(k, smem);
+  e = set_smem(k, smem);
   if (e != cudaSuccess) return e;
   int per = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, 256, smem);

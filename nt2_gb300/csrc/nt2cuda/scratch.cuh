@@ -5,10 +5,13 @@
 // different streams never share scratch; calls on one stream are ordered and
 // reuse it.  A buffer only grows; growing synchronises its stream first.  The
 // first call on a stream allocates (cudaMalloc), so make it before capturing
-// that stream into a CUDA graph.  The folds' arrival counters have a slot of
-// their own: they start at zero (a buffer is cleared when allocated), every
-// fold leaves the ones it used at zero, and nothing else is written there --
-// partials, which other kernels overwrite freely, live in another slot.
+// that stream into a CUDA graph.  A graph keeps the addresses, so its launches
+// have to be ordered with the calls and graphs that share them (captured folds
+// of columns of up to 4096 16-byte groups use none).  The folds' arrival
+// counters have a slot of their own: they start at zero (a buffer is cleared
+// when allocated), every fold leaves the ones it used at zero, and nothing else
+// is written there -- partials, which other kernels overwrite freely, live in
+// another slot.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -29,17 +32,23 @@ inline scratch_pool& global_scratch_pool() { static scratch_pool p; return p; }
 // descriptors, scan flags and carries); slot 2: fold partials; slot 3
 // (kResultSlot): device results the C++ front end reads back (globalsum).
 constexpr int kResultSlot = 3;
-inline cudaError_t stream_scratch(cudaStream_t s, size_t bytes, void** out, int slot = 0);
+inline cudaError_t stream_scratch(cudaStream_t s, size_t bytes, void** out, int slot = 0, size_t room = 0);
 
-// The two buffers of a fold: ncounters zero-valued arrival counters and room
-// for npartials partial states of `partial_bytes` each.
-inline cudaError_t fold_scratch(cudaStream_t s, size_t ncounters, size_t npartials, size_t partial_bytes,
-                                unsigned** counters, void** partials)
+// The two buffers of a fold of n outputs, each cut into `splits` segments: a
+// zero-valued arrival counter and splits * states partial states of `partial_bytes`
+// for each output (none where it is not cut).  Outside capture they are made large
+// enough for `wide` segments too, the cut of a captured call.
+inline cudaError_t fold_scratch(cudaStream_t s, size_t n, size_t splits, size_t wide, size_t partial_bytes,
+                                unsigned** counters, void** partials, size_t states = 1)
 {
+  const size_t most = splits > wide ? splits : wide;
   void* c = nullptr;
-  cudaError_t e = stream_scratch(s, ncounters * sizeof(unsigned), &c, 0);
+  *counters = nullptr;
+  *partials = nullptr;
+  if (most <= 1) return cudaSuccess;
+  cudaError_t e = stream_scratch(s, splits > 1 ? n * sizeof(unsigned) : 0, &c, 0, n * sizeof(unsigned));
   if (e != cudaSuccess) return e;
-  e = stream_scratch(s, npartials * partial_bytes, partials, 2);
+  e = stream_scratch(s, splits > 1 ? n * splits * states * partial_bytes : 0, partials, 2, n * most * states * partial_bytes);
   *counters = (unsigned*)c;
   return e;
 }
@@ -51,34 +60,32 @@ inline uintptr_t scratch_key(cudaStream_t s, int slot)
   return (reinterpret_cast<uintptr_t>(s) * 64u + (uintptr_t)dev) * 4u + (uintptr_t)slot;
 }
 
-// Whether a fold's buffers could not be had now: they would have to be
-// allocated, and the stream is being captured.
-inline bool fold_scratch_barred(cudaStream_t s, size_t ncounters, size_t npartials, size_t partial_bytes)
+// Whether the stream is being captured into a CUDA graph.
+inline bool capturing(cudaStream_t s)
 {
-  {
-    scratch_pool& P = global_scratch_pool();
-    const uintptr_t k0 = scratch_key(s, 0), k2 = scratch_key(s, 2);
-    std::lock_guard<std::mutex> g(P.m);
-    if (P.by_key[k0].bytes >= ncounters * sizeof(unsigned) && P.by_key[k2].bytes >= npartials * partial_bytes) return false;
-  }
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-  return cudaStreamIsCapturing(s, &st) == cudaSuccess && st != cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &st) == cudaSuccess) return st != cudaStreamCaptureStatusNone;
+  (void)cudaGetLastError();
+  return false;
 }
 
-inline cudaError_t stream_scratch(cudaStream_t s, size_t bytes, void** out, int slot)
+// At least `bytes`; a buffer that grows, and outside capture one smaller than
+// `room`, becomes the larger of the two.
+inline cudaError_t stream_scratch(cudaStream_t s, size_t bytes, void** out, int slot, size_t room)
 {
   const uintptr_t key = scratch_key(s, slot);
   scratch_pool& P = global_scratch_pool();
   std::lock_guard<std::mutex> g(P.m);
   scratch_pool::entry& e = P.by_key[key];
-  if (e.bytes < bytes) {
+  if (room < bytes) room = bytes;
+  if (e.bytes < room && (e.bytes < bytes || !capturing(s))) {
     if (e.p) {
       cudaStreamSynchronize(s);
       cudaFree(e.p);
       e.p = nullptr;
       e.bytes = 0;
     }
-    size_t want = bytes < 4096 ? 4096 : bytes;
+    size_t want = room < 4096 ? 4096 : room;
     cudaError_t err = cudaMalloc(&e.p, want);
     if (err != cudaSuccess) { e.p = nullptr; return err; }
     ++P.allocations;
