@@ -7,7 +7,9 @@
 // first call on a stream allocates (cudaMalloc), so make it before capturing
 // that stream into a CUDA graph.  A graph keeps the addresses, so its launches
 // have to be ordered with the calls and graphs that share them (captured folds
-// of columns of up to 4096 16-byte groups use none).  The folds' arrival
+// of columns of up to 4096 16-byte groups use none), and a buffer that a larger
+// one replaces stays allocated: the larger one is at least twice its size, so
+// those before the last take less than it together.  The folds' arrival
 // counters have a slot of their own: they start at zero (a buffer is cleared
 // when allocated), every fold leaves the ones it used at zero, and nothing else
 // is written there -- partials, which other kernels overwrite freely, live in
@@ -79,18 +81,18 @@ inline cudaError_t stream_scratch(cudaStream_t s, size_t bytes, void** out, int 
   scratch_pool::entry& e = P.by_key[key];
   if (room < bytes) room = bytes;
   if (e.bytes < room && (e.bytes < bytes || !capturing(s))) {
-    if (e.p) {
-      cudaStreamSynchronize(s);
-      cudaFree(e.p);
-      e.p = nullptr;
-      e.bytes = 0;
-    }
-    size_t want = room < 4096 ? 4096 : room;
-    cudaError_t err = cudaMalloc(&e.p, want);
-    if (err != cudaSuccess) { e.p = nullptr; return err; }
-    ++P.allocations;
-    err = cudaMemsetAsync(e.p, 0, want, s);
+    cudaError_t err = e.p ? cudaStreamSynchronize(s) : cudaSuccess;   // (an error under capture)
     if (err != cudaSuccess) return err;
+    size_t want = room < 4096 ? 4096 : room;
+    if (want < 2 * e.bytes) want = 2 * e.bytes;
+    void* p = nullptr;
+    if ((err = cudaMalloc(&p, want)) != cudaSuccess) return err;
+    ++P.allocations;
+    if ((err = cudaMemsetAsync(p, 0, want, s)) != cudaSuccess) {
+      cudaFree(p);
+      return err;
+    }
+    e.p = p;
     e.bytes = want;
   }
   *out = e.p;

@@ -113,6 +113,30 @@ def test_graph_outlives_the_scratch_of_its_stream(gpu, cuda_lib, op, rows, cols,
     check(op, out, A, rows, cols, dim)
 
 
+@pytest.mark.parametrize("dim", [1, 2])
+def test_graph_keeps_the_scratch_it_holds(gpu, cuda_lib, dim):
+    """A captured fold that does use scratch still writes its own after a larger fold on the
+    stream has made that grow."""
+    rows, cols = (200000, 3) if dim == 1 else (3, 200000)
+    A, big = table(rows * cols, torch.float32, 5), table(1 << 21, torch.float32, 1)
+    out = torch.zeros(m_of(rows, cols, dim), device="cuda")
+    with own_stream() as s:
+        warm(s, "sum", A, rows, cols, dim)
+        g = capture(s, "sum", A, rows, cols, dim, out)
+        n = allocations(cuda_lib)
+        warm(s, "sum", big, 512, 4096, 2)
+        assert allocations(cuda_lib) > n
+        other = torch.full((1 << 20,), 3.0, device="cuda")            # what a freed buffer would be handed out as
+        g.replay()
+        torch.cuda.synchronize()
+        assert bool((other == 3.0).all())
+        check("sum", out, A, rows, cols, dim)
+        with torch.cuda.stream(s):
+            got = api.reduce("sum", big, 512, 4096, dim=2, compensated=False)
+        s.synchronize()
+    check("sum", got, big, 512, 4096, 2)
+
+
 # the fold that warms the stream, and one whose partials (one for every 4096 16-byte groups of a
 # column, or for every 64 to 128 columns of a strip of rows) fit what that allocated
 FITS = [(("sum", 40000, 1, 1, 0), ("sum", 20000, 100, 1, 0), torch.float32),
