@@ -92,22 +92,23 @@ inline int sm_count()
 
 // Blocks of a kernel that fit one SM.  The query takes a tenth of a small call,
 // so each thread keeps the answers of the kernels it launches (they depend on
-// the kernel, the block and the device alone).
-template <class K> inline int resident_blocks(K kernel, int block)
+// the kernel, the block and the device alone), in one table of 6 KB whatever
+// the kernels' types.
+inline int resident_blocks_of(const void* f, int block)
 {
   struct entry { const void* f; int block, dev, nb; };
   constexpr unsigned N = 256;
   static thread_local entry cache[N] = {};
   int dev = 0;
   cudaGetDevice(&dev);
-  const void* f = (const void*)kernel;
   entry& e = cache[((uintptr_t)f >> 4 ^ (uintptr_t)f >> 12 ^ (uintptr_t)block) % N];
   if (e.f == f && e.block == block && e.dev == dev) return e.nb;
   int nb = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, block, 0) != cudaSuccess || nb < 1) return 1;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, f, block, 0) != cudaSuccess || nb < 1) return 1;
   e = entry{f, block, dev, nb};
   return nb;
 }
+template <class K> inline int resident_blocks(K kernel, int block) { return resident_blocks_of((const void*)kernel, block); }
 
 // Launch as a programmatic dependent of the previous kernel on the stream:
 // the grid may be scheduled while its predecessor finishes, and waits in
