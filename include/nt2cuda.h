@@ -586,7 +586,8 @@ nt2cuda_status nt2cuda_server_replay(nt2cuda_server* server, const float* S, con
  * "saxpy_f64", "bs_f32", "bs_f32_fused", "bs_f32_fast", "bs_f64",
  * "bs_f64_fused" (the Black-Scholes keys are per precision mode), and
  * "bs_f32_mapped", "bs_f32_fast_mapped" (the kernel on pinned host tables,
- * as nt2cuda_blackscholes_f32_host runs it), "rgb2grey_u8". */
+ * as nt2cuda_blackscholes_f32_host runs it), "rgb2grey_u8".  The double
+ * Black-Scholes kernel has one unroll: its keys are tuned for the waves only. */
 nt2cuda_status nt2cuda_autotune(const char* kernel, size_t n, int* best_unroll, int* best_waves, float* best_ms);
 /* Tuning table as text ("key@bucket unroll waves" lines). */
 nt2cuda_status nt2cuda_tuning_export(char* buf, size_t cap, size_t* needed);

@@ -207,10 +207,11 @@ nt2cuda_status bs_launch(const T* S, const T* K, const T* Tm, T r, T v, T* call,
   if (n == 0) return NT2CUDA_OK;
   size_t nn = n;
   void* args[] = {(void*)&S, (void*)&K, (void*)&Tm, (void*)&r, (void*)&v, (void*)&call, (void*)&put, (void*)&nn};
-  const bool vec = sizeof(T) == 4 && aligned16(S) && aligned16(K) && aligned16(Tm) && aligned16(call) && aligned16(put);
-  if (!vec)
-    return launch_status(launch_persistent(k_blackscholes_scalar<T, CDF, P>, n, sizeof(T) == 8 ? f64_block(n) : 256, waves, s, args));
-  if constexpr (sizeof(T) == 4) {
+  if constexpr (sizeof(T) == 8) {       // one kernel, whatever `unroll` (see one_group in expr.cuh)
+    return launch_status(launch_persistent(k_blackscholes_scalar<T, CDF, P>, n, f64_block(n), waves, s, args));
+  } else {
+    if (!(aligned16(S) && aligned16(K) && aligned16(Tm) && aligned16(call) && aligned16(put)))
+      return launch_status(launch_persistent(k_blackscholes_scalar<T, CDF, P>, n, 256, waves, s, args));
     size_t groups = n / 4;
     switch (unroll) {
       case 1: return launch_status(launch_persistent(k_blackscholes<T, CDF, P, 1>, groups, 256, waves, s, args));
@@ -218,7 +219,6 @@ nt2cuda_status bs_launch(const T* S, const T* K, const T* Tm, T r, T v, T* call,
       default: return launch_status(launch_persistent(k_blackscholes<T, CDF, P, 2>, groups, 256, waves, s, args));
     }
   }
-  return NT2CUDA_ERR_ARG;
 }
 
 template <class T, int CDF>
@@ -533,11 +533,12 @@ nt2cuda_status nt2cuda_autotune(const char* kernel, size_t n, int* best_unroll, 
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
   const int unrolls[3] = {1, 2, 4};
+  const int variants = bs64 ? 1 : 3;                     // the double kernel has one
   const int wavesv[4] = {1, 2, 4, 8};
   float best = 1e30f;
   tuning::params bp;
   nt2cuda_status st = NT2CUDA_OK;
-  for (int ui = 0; ui < 3 && st == NT2CUDA_OK; ++ui)
+  for (int ui = 0; ui < variants && st == NT2CUDA_OK; ++ui)
     for (int wi = 0; wi < 4 && st == NT2CUDA_OK; ++wi) {
       auto once = [&]() -> nt2cuda_status {
         if (bs32)
