@@ -363,8 +363,7 @@ template <int SH> NT2_F64I int64_t to_fixed(double x, uint32_t F)
   const int64_t v = (int64_t)shr64(m, F - ((h >> 20) & 0x7ffu));
   return (int32_t)h < 0 ? -v : v;
 }
-// largest biased exponent of a block; frames are made for 64 <= F < 2000 (no
-// infinities or NaNs, and the unit a normal number)
+// largest biased exponent of a block
 template <int N> NT2_F64I uint32_t max_exponent(const double (&x)[N])
 {
   uint32_t m = 0u;
@@ -375,12 +374,5 @@ template <int N> NT2_F64I uint32_t max_exponent(const double (&x)[N])
   }
   return m >> 20;
 }
-NT2_F64I bool frame_range(uint32_t F) { return F - 64u < 2000u - 64u; }
-// v * 2^n rounded to nearest; v an integer, 2^n and the product normal
-NT2_F64I double from_fixed(int64_t v, int n)
-{
-  return v ? scale((double)v, n) : 0.0;
-}
-
 }  // namespace f64i
 }  // namespace nt2cuda
