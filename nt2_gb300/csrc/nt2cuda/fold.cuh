@@ -350,15 +350,71 @@ template <int FIN, class E> struct block_acc<op_sum<false, FIN>, double, E> {
   }
 };
 
+// Count, mean and M2 of n values in a fixed point frame of unit 2^(F - 1075 - SH),
+// from a pivot P and the exact sums s of d = value - P (128 bits) and q of d^2 (192):
+// M2 = q - s^2/n.  The pivot is a few values' mean, and q may be far above M2 (n/N
+// times, for the mean of N values that the rest are far from); where M2 is less than
+// a quarter of q, frame_recentred moves the sums first.
+template <int SH>
+__device__ __forceinline__ moments<double> frame_result(double cnt, uint32_t F, int64_t P, double md, double m2)
+{
+  const double unit = f64i::from_bits((uint64_t)(F - 1075u - (uint32_t)SH + 1023u) << 52);
+  return moments<double>{cnt, ((double)P + md) * unit, fmax(m2, 0.0) * unit * unit};
+}
+constexpr double kTwo64 = 18446744073709551616.0;
+// To c, the mean of d rounded to a whole unit or nearly, while the sums are integers:
+// s - n c and q - c (s + (s - n c)).  What is left cancels nothing.
+template <int SH>
+__device__ __forceinline__ moments<double> frame_recentred(int n, uint32_t F, int64_t P, int64_t s_hi, uint64_t s_lo, uint64_t q_x,
+                                                        uint64_t q_hi, uint64_t q_lo)
+{
+  const double cnt = (double)n;
+  const int64_t c = __double2ll_rn(math::div(__fma_rn((double)s_hi, kTwo64, (double)s_lo), cnt));
+  const int64_t r = (int64_t)(s_lo - (uint64_t)n * (uint64_t)c);         // s - n c, 2^8 n at most
+  uint64_t v_lo = s_lo + (uint64_t)r;
+  uint64_t v_hi = (uint64_t)(s_hi + (r >> 63) + (v_lo < s_lo ? 1 : 0));
+  const bool vn = (int64_t)v_hi < 0, cn = c < 0;
+  if (vn) {
+    v_hi = ~v_hi + (v_lo == 0ull ? 1ull : 0ull);
+    v_lo = 0ull - v_lo;
+  }
+  const uint64_t u = cn ? 0ull - (uint64_t)c : (uint64_t)c;
+  const unsigned __int128 p0 = (unsigned __int128)u * v_lo, p1 = (unsigned __int128)u * v_hi + (uint64_t)(p0 >> 64);
+  uint64_t w0 = (uint64_t)p0, w1 = (uint64_t)p1, w2 = (uint64_t)(p1 >> 64);
+  if (vn == cn) {                                                         // q - w as q + ~w + 1
+    w0 = ~w0;
+    w1 = ~w1;
+    w2 = ~w2;
+  }
+  const unsigned __int128 a0 = (unsigned __int128)q_lo + w0 + (vn == cn ? 1u : 0u);
+  const unsigned __int128 a1 = (unsigned __int128)q_hi + w1 + (uint64_t)(a0 >> 64);
+  const uint64_t a2 = q_x + w2 + (uint64_t)(a1 >> 64);
+  const double q = __fma_rn(__fma_rn((double)a2, kTwo64, (double)(uint64_t)a1), kTwo64, (double)(uint64_t)a0);
+  const double rd = (double)r, md = math::div(rd, cnt);
+  return frame_result<SH>(cnt, F, P + c, md, __fma_rn(-rd, md, q));
+}
+template <int SH>
+__device__ __forceinline__ moments<double> frame_moments(int n, uint32_t F, int64_t P, int64_t s_hi, uint64_t s_lo, uint32_t q_x,
+                                                         uint64_t q_hi, uint64_t q_lo)
+{
+  const double cnt = (double)n;
+  const bool neg = s_hi < 0;
+  const uint64_t lo = neg ? 0ull - s_lo : s_lo;
+  const uint64_t hi = neg ? ~(uint64_t)s_hi + (s_lo == 0ull ? 1ull : 0ull) : (uint64_t)s_hi;
+  const double mag = __fma_rn((double)hi, kTwo64, (double)lo), q = __fma_rn(__fma_rn((double)q_x, kTwo64, (double)q_hi), kTwo64, (double)q_lo);
+  const double md = math::div(mag, cnt), m2 = __fma_rn(-mag, md, q);
+  // m2 below a quarter of q, or negative (the bits compare as integers)
+  if ((int64_t)f64i::bits(m2) + (2ll << 52) < (int64_t)f64i::bits(q)) return frame_recentred<SH>(n, F, P, s_hi, s_lo, q_x, q_hi, q_lo);
+  return frame_result<SH>(cnt, F, P, neg ? -md : md, m2);
+}
+
 // var / stdev of doubles: the lane keeps its values' sum and their squared
 // distances from a pivot P (the first block's mean) as exact integers in one
 // fixed point frame, two bits above the first block's largest exponent.  A
 // value costs some 28 integer instructions and no double ones (three on the
 // double pipe, 48 clocks a warp, in the blockwise two-pass form); a value
-// beyond the frame, or 512 values, closes it: its count, mean and M2 =
-// sum d^2 - (sum d)^2/n become doubles and merge into the state.  P is one of
-// n <= 512 values' block means, so (sum d)^2/n is at most about n/16 times M2
-// and the subtraction loses no more than a few bits in the worst case.
+// beyond the frame, or 512 values, closes it: its count, mean and M2 become
+// doubles (frame_moments) and merge into the state.
 template <bool W1, bool SD, class E> struct block_acc<op_moments<W1, SD>, double, E> {
   static constexpr bool value = true;
   using Op = op_moments<W1, SD>;
@@ -419,10 +475,6 @@ template <bool W1, bool SD, class E> struct block_acc<op_moments<W1, SD>, double
     q_hi += hi + (t < lo ? 1ull : 0ull);
     q_lo = t;
   }
-  __device__ __forceinline__ static double to_double(uint64_t hi, uint64_t lo)
-  {
-    return __fma_rn((double)hi, 18446744073709551616.0, (double)lo);
-  }
   __device__ __forceinline__ void flush(S& a)
   {
     if (n) a = closed(a, n, F, P, s_hi, s_lo, q_hi, q_lo);
@@ -431,15 +483,7 @@ template <bool W1, bool SD, class E> struct block_acc<op_moments<W1, SD>, double
   static __device__ __noinline__ S closed(S a, int n, uint32_t F, int64_t P, int64_t s_hi, uint64_t s_lo, uint64_t q_hi,
                                           uint64_t q_lo)
   {
-    const double cnt = (double)n;
-    const bool neg = s_hi < 0;
-    const uint64_t lo = neg ? 0ull - s_lo : s_lo;
-    const uint64_t hi = neg ? ~(uint64_t)s_hi + (s_lo == 0ull ? 1ull : 0ull) : (uint64_t)s_hi;
-    const double sd = neg ? -to_double(hi, lo) : to_double(hi, lo);        // sum of (value - P)
-    const double md = math::div(sd, cnt);
-    const double m2 = fmax(__fma_rn(-sd, md, to_double(q_hi, q_lo)), 0.0);
-    const double unit = f64i::from_bits((uint64_t)(F - 1075u - (uint32_t)SH + 1023u) << 52);
-    return Op::merge(a, S{cnt, ((double)P + md) * unit, m2 * unit * unit});
+    return Op::merge(a, frame_moments<SH>(n, F, P, s_hi, s_lo, 0u, q_hi, q_lo));
   }
 };
 
@@ -570,16 +614,7 @@ template <class Op, int N> struct warp_frame {
       q_x += qx + (h1 < qh ? 1u : 0u) + (h2 < c ? 1u : 0u);
       q_hi = h2;
     }
-    const double two64 = 18446744073709551616.0, cnt = (double)n;
-    const bool neg = s_hi < 0;
-    const uint64_t lo = neg ? 0ull - s_lo : s_lo;
-    const uint64_t hi = neg ? ~(uint64_t)s_hi + (s_lo == 0ull ? 1ull : 0ull) : (uint64_t)s_hi;
-    const double mag = __fma_rn((double)hi, two64, (double)lo), sd = neg ? -mag : mag;    // sum of (value - P)
-    const double q = __fma_rn(__fma_rn((double)q_x, two64, (double)q_hi), two64, (double)q_lo);
-    const double md = math::div(sd, cnt);
-    const double m2 = fmax(__fma_rn(-sd, md, q), 0.0);
-    const double unit = f64i::from_bits((uint64_t)(F - 1075u - (uint32_t)SH + 1023u) << 52);
-    return Op::merge(a, S{cnt, ((double)P + md) * unit, m2 * unit * unit});
+    return Op::merge(a, frame_moments<SH>(n, F, P, s_hi, s_lo, q_x, q_hi, q_lo));
   }
 };
 template <class Op, class T> struct warp_framed { static constexpr bool value = false; };
