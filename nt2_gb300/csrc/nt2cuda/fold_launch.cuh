@@ -32,13 +32,13 @@ template <class E> bool expr_aligned(const E& e)
 // How inner_fold cuts columns into segments, one to a warp: into about
 // `kInnerUnits` segments in all, 24 a SM with 16-byte loads and 16 with single
 // elements, so that a few long columns fill the chip too (3333333 x 1 floats:
-// 44 us with segments of 16384, 10.5 with 2432 of them), but never below eight
+// 44 us with segments of 16384, 10.5 with 16 a SM), but never below eight
 // loads a lane, and at most kInnerSplits to a column, as one warp merges them.
 // The cut depends on the table's shape alone (and on whether the call is captured,
 // see captured_cut): results are reproducible.
 // (var/stdev of doubles: 16 a SM in either case, what their 128 registers leave
 // room for; 70000 x 111: 46.9 us with 8, 40.7 with 16, 41.6 with 24.)
-constexpr size_t kInnerUnits = 3648, kInnerUnitsScalar = 2432, kInnerSplits = 2432;
+constexpr size_t kInnerUnits = 24 * kSms, kInnerUnitsScalar = 16 * kSms, kInnerSplits = 16 * kSms;
 template <class Op, class T> inline size_t inner_seg(size_t rows, size_t cols, bool vec)
 {
   const size_t lanes = vec ? 32 * (16 / sizeof(T)) : 32;
@@ -77,7 +77,7 @@ template <class T> inline const T* first_term(const node<tag::multiplies_, term<
 template <class T> inline const T* second_term(const term<T>&) { return nullptr; }
 template <class T> inline const T* second_term(const node<tag::multiplies_, term<T>, term<T>>& n) { return n.b.p; }
 
-// Loads in flight per lane in the register-pipelined kernels: 16, or 8 where a
+// Loads of a lane's trip in the register-pipelined kernels: 16, or 8 where a
 // trip's values form a block (block_acc): its values stay in registers.
 template <class Op, class T, class E> struct fold_unroll {
   static constexpr int value = block_acc<Op, T, E>::value ? 8 : 16;
@@ -86,9 +86,9 @@ template <class Op, class T, class E> struct fold_unroll {
 template <class Op, class T, class E> struct outer_unroll { static constexpr int value = fold_unroll<Op, T, E>::value; };
 template <bool W1, bool SD, class E> struct outer_unroll<op_moments<W1, SD>, float, E> { static constexpr int value = 4; };
 // Tables whose rows or alignment rule out 16-byte loads: one element per lane
-// and load, so as many loads in flight again.
+// and load, so 16 loads a trip again.
 constexpr int kScalarUnroll = 16;
-constexpr size_t kOuterUnits = 608;
+constexpr size_t kOuterUnits = 4 * kSms;
 
 // Segments of inner_fold under capture (captured_cut): 128 loads of 16 bytes a lane,
 // or 16 bulk-copy tiles where a column of double var/stdev would otherwise be staged.
@@ -154,7 +154,7 @@ cudaError_t inner_fold(const E& e, size_t rows, size_t cols, out_of<Op, T>* out,
   out_of<Op, T>* o = out;
   void* args[] = {&ec, &sh, &o, &partials, &counters};
   // launch_persistent counts threads; a unit is one warp.  Columns of at most
-  // eight loads a lane take the kernel with four in flight.
+  // eight loads a lane take the kernel with four a trip.
   if (rows <= (size_t)32 * (vec ? VV : 1) * 8) {
     if (vec) return (launch_persistent(k_inner<Op, VV, 4, T, E>, units * 32, 128, 4, s, args));
     return (launch_persistent(k_inner<Op, 1, 4, T, E>, units * 32, 128, 4, s, args));
@@ -186,7 +186,7 @@ cudaError_t outer_fold(const E& e, size_t rows, size_t cols, out_of<Op, T>* out,
   sh.rows = rows;
   sh.cols = cols;
   sh.strips = (rows + STRIP - 1) / STRIP;
-  // as many chunks as keep the blocks within 608, four a SM: one wave, every
+  // as many chunks as keep the blocks within four a SM: one wave, every
   // block at once (8192 x 4096 floats in 640 blocks takes 29.8 us); under capture
   // (captured_cut) whole 64 columns in about 512 blocks.  The split depends only on
   // the shape, so results stay reproducible.

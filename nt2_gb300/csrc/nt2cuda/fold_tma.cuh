@@ -87,17 +87,17 @@ struct inner_tma_shape {
   uint32_t wait_rounds;
 };
 
-// Elements of a unit.  The blocks are resident all at once (2 a SM of 152 with
+// Elements of a unit.  The blocks are resident all at once (2 a SM with
 // two tables, 3 with one) and stream one tile after another, so the longest
 // block's elements decide: the columns are cut into the number of segments, of
 // the candidates that give every block 1, 2, ... 8 of them, with the fewest
 // elements to a block, half a tile counted for each unit's start and end.
-// (dot over 2^26 floats: 91.5 us in 1024 units of 16 tiles, 80.0 in 304;
-// 4000000 floats: 17.7 us in 62 units, 7.8 in 456.)  At least a quarter tile.
+// (dot over 2^26 floats: 91.5 us in 1024 units of 16 tiles, 80.0 in 2 a SM;
+// 4000000 floats: 17.7 us in 62 units, 7.8 in 3 a SM.)  At least a quarter tile.
 template <class T> inline size_t inner_tma_seg(size_t rows, size_t cols, int tables)
 {
   constexpr size_t TILE = kTmaTileBytes / sizeof(T), VV = 16 / sizeof(T);
-  const size_t slots = tables == 2 ? 304 : 456;
+  const size_t slots = (tables == 2 ? 2 : 3) * kSms;
   size_t best = rows, best_cost = ~(size_t)0;
   for (size_t k = 1; k <= 8; ++k) {
     const size_t per_col = k * slots / cols > 1 ? k * slots / cols : 1;

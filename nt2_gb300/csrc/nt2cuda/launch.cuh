@@ -78,6 +78,9 @@ template <class P> inline bool all_aligned(const P& p, unsigned align)
 }
 
 // ----------------------------------------------------------- launching
+// SMs of a GB300.  Tables are cut by this number, not by the device's own, so that
+// results depend on their shape alone.
+constexpr size_t kSms = 152;
 inline int sm_count()
 {
   static int sms = 0;

@@ -719,7 +719,7 @@ __global__ void __launch_bounds__(256, (scan_min_blocks<Op, T>::value)) k_scan_i
 // the SM's issue slots at full bandwidth, so the gathering warps' work is
 // kept short: four lanes share a tile's digits, so that a tile is one 16-byte
 // load and four additions in each, and the pair is made from the digits as floats.
-// The warps share the 152 or so tiles of a gather, so that its loads are in flight
+// The warps share a gather's tiles, one for each SM or so, so that its loads are in flight
 // at once: 2^26 floats 106 us with one or two warps, 102.6 with three of seven loads
 // a lane, 100.1 with five of four.)
 // 2^26 floats: 101 us, 78% of a copy of the same bytes (79 us); the two-pass tiles

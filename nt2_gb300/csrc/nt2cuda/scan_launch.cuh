@@ -27,10 +27,10 @@ template <class Op, class T> inline size_t lookback_scratch(size_t tiles)
 
 // The streamed scan of long float columns (k_scan_stream).  cudaErrorNotSupported,
 // before anything is launched, when it does not apply.
-// At least a tile for each of 152 SMs (1.9 million floats 18.2 us before, 15.1),
-// and the columns' last tiles at least an eighth of a column full in all
+// At least a tile for each SM (1.9 million floats 18.2 us before, 15.1),
+// and at most an eighth of padding in the columns' last tiles
 // (16384 x 1000, a third of whose tiles' rows would be padding: 39.7 against 50).
-constexpr size_t kStreamTiles = 152;
+constexpr size_t kStreamTiles = kSms;
 template <class Op, class T> struct streamed { static constexpr bool value = false; };
 template <bool COMP> struct streamed<fold::op_sum<COMP>, float> { static constexpr bool value = true; static constexpr bool comp = COMP; };
 // first, wait_rounds and polls are for the timeout self-test: the tile handed out
