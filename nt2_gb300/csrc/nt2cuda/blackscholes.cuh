@@ -268,9 +268,9 @@ __global__ void __launch_bounds__(256, U == 1 ? 4 : 3)
 }
 
 // One option per thread per trip: misaligned tables, and doubles (aligned or
-// not: see one_group in expr.cuh; 2^24 options 2.89 ms at the 64 registers of
-// four blocks per SM, where the double pipe, 90 instructions an option, would
-// allow 2.55).
+// not: see one_group in expr.cuh; 2^24 options 2.93 ms at the 64 registers of
+// four blocks per SM, where the double pipe, 87 instructions an option, would
+// allow 2.5).
 template <class T, int CDF, int P>
 __global__ void __launch_bounds__(256, sizeof(T) == 8 ? 4 : 0) k_blackscholes_scalar(const T* S, const T* K, const T* Tm, T r, T v,
                                                              T* call, T* put, size_t n)

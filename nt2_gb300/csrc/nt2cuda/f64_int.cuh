@@ -8,8 +8,10 @@
 // dependent chains the multiply below reaches 2.6 per clock and SM, the
 // division 1.1 and the root 1.1, and they run beside the additions, which stay
 // on the double pipe: multiply and add together 1.85 per clock against 0.95
-// for the two instructions.  2^24 exact Black-Scholes options in double went
-// from 12.35 to 6.47 ms, sin over 3000001 doubles from 256 to 159 us.
+// for the two instructions.  2^24 exact Black-Scholes options in double take
+// 2.93 ms (12.35 with the double instructions; 6.47 with these forms in the
+// functors as they were written for those), sin over 3000001 doubles 79 us (256,
+// 159).
 //
 // Results are the IEEE round-to-nearest-even ones, bit for bit.  The integer
 // form covers operands whose exponents keep every intermediate normal; the

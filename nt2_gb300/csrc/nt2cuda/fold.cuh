@@ -680,10 +680,10 @@ struct inner_shape {
   size_t rows, cols, seg, splits;
 };
 
-// fold_min_blocks: left to itself the
-// compiler keeps 48 registers, 32 where a lane loads single elements, and
-// issues the U loads a few at a time (sum(A,1) of 8192 x 4096 floats 24.5 us,
-// now 21.5; 300001 x 50, single elements, 27.8 us, now 14.8).
+// fold_min_blocks: left to itself the compiler keeps 48 registers, 32 where a
+// lane loads single elements; 64 leave room for more of a trip's loads at once
+// (though not for all of 16 times 16 bytes): sum(A,1) of 8192 x 4096 floats
+// 24.5 us, now 21.5; 300001 x 50, single elements, 27.8 us, now 14.8.
 template <class Op, int V, int U, class T, class E>
 __global__ void __launch_bounds__(256, (fold_min_blocks<Op, T, U>::value)) k_inner(E e, inner_shape sh, out_of<Op, T>* __restrict__ out,
                                                state_of<Op, T>* __restrict__ partials, unsigned* __restrict__ counters)
@@ -891,9 +891,8 @@ struct outer_shape {
   size_t rows, cols, cchunk, splits, strips;
 };
 
-// fold_min_blocks: left to itself the compiler keeps 48 registers
-// (32 where a lane loads single elements) and issues the U loads a few at a time
-// (8192 x 4096 floats 24.2 us, now 22.5; 10001 x 777 floats 20.3, now 9.7).
+// fold_min_blocks: as in k_inner (8192 x 4096 floats 24.2 us with the compiler's
+// own 48 registers, now 22.5; 10001 x 777 floats 20.3, now 9.7).
 template <class Op, int V, int U, class T, class E>
 __global__ void __launch_bounds__(256, (fold_min_blocks<Op, T, U>::value)) k_outer(E e, outer_shape sh, out_of<Op, T>* __restrict__ out,
                                                state_of<Op, T>* __restrict__ partials, unsigned* __restrict__ counters)

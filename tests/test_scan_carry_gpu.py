@@ -100,3 +100,14 @@ def test_subnormals_and_non_finite(gpu, cuda_lib, name, tile, offset, compensate
     assert np.isfinite(got[:100 * tile + 5]).all()
     assert np.isposinf(got[100 * tile + 5:190 * tile + 9]).all()
     assert np.isnan(got[190 * tile + 9:]).all()
+
+
+@pytest.mark.parametrize("compensated", [True, False])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_long_column_is_reproducible(gpu, cuda_lib, offset, compensated):
+    """2^24 elements, streamed or chained through the look-back: the same bits each time."""
+    a = np.random.default_rng(6).standard_normal(1 << 24).astype(np.float32)
+    got = cumsum(a, offset, compensated)
+    assert np.array_equal(got, cumsum(a, offset, compensated))
+    ref, mag = np.cumsum(a.astype(np.float64)), np.cumsum(np.abs(a.astype(np.float64)))
+    assert np.all(np.abs(got - ref) <= bound(ref, mag, compensated))
