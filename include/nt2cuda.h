@@ -339,8 +339,11 @@ nt2cuda_status nt2cuda_blackscholes_f32_host(const float* S, const float* K, con
  * demo/sdot/nt2/sdot_nt2.cpp:35-38): the inner_fold over one column of n
  * elements.  *out is a DEVICE scalar.  compensated = 1 accumulates FP32 with
  * TwoSum-compensated partials; 0 is the plain tree sum.  The block
- * decomposition depends only on n, so results are bitwise reproducible.
- * The first call on a stream allocates that stream's scratch. */
+ * decomposition depends only on n, and on whether the stream is being captured
+ * into a graph, so results are bitwise reproducible.  The first call on a stream
+ * allocates that stream's scratch; a graph whose folds use it (columns of more
+ * than 4096 16-byte groups, row sums of more than 64 columns) may not run at the
+ * same time as other work or graphs of the stream it was captured on. */
 nt2cuda_status nt2cuda_globalsum_f32(const float* x, size_t n, float* out, int compensated, nt2cuda_stream stream);
 nt2cuda_status nt2cuda_dot_f32(const float* x, const float* y, size_t n, float* out, int compensated,
                                nt2cuda_stream stream);

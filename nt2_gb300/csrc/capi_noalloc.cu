@@ -35,7 +35,7 @@ using nt2cuda::fold::acc;
 
 namespace {
 
-constexpr size_t kSeg = (size_t)32 * 4 * 128;                         // a warp's segment, as nt2cuda_dot_f32
+constexpr size_t kSeg = (size_t)32 * 4 * 128;                         // a warp's segment
 constexpr size_t kMaxSplits = (size_t)NT2CUDA_DOT_NOALLOC_MAX_N / kSeg;
 constexpr size_t kCounterBytes = 256;
 constexpr size_t kScratchBytes = kCounterBytes + kMaxSplits * sizeof(acc<float>);

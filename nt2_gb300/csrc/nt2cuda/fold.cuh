@@ -14,8 +14,8 @@
 // Here the element values come from an expression (so globalsum(X*Y) reads X
 // and Y once, as NT2's fused fold_step does), FP32 accumulates with
 // TwoSum-compensated partials when COMP is set, and the split of the work
-// into warps and blocks depends only on the table's shape: partials are
-// combined in index order, never in arrival order, so results are bitwise
+// into warps and blocks depends only on the table's shape (and on whether the
+// call is captured into a graph, captured_cut): partials are combined in index order, never in arrival order, so results are bitwise
 // reproducible from run to run and across GPUs.
 #pragma once
 #include <cuda_runtime.h>
