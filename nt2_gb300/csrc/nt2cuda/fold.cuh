@@ -15,8 +15,9 @@
 // and Y once, as NT2's fused fold_step does), FP32 accumulates with
 // TwoSum-compensated partials when COMP is set, and the split of the work
 // into warps and blocks depends only on the table's shape (and on whether the
-// call is captured into a graph, captured_cut): partials are combined in index order, never in arrival order, so results are bitwise
-// reproducible from run to run and across GPUs.
+// call is captured into a graph, captured_cut): partials are combined in index
+// order, never in arrival order, so results are bitwise reproducible from run to
+// run and across GPUs.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -414,7 +415,10 @@ __device__ __forceinline__ moments<double> frame_moments(int n, uint32_t F, int6
 // value costs some 28 integer instructions and no double ones (three on the
 // double pipe, 48 clocks a warp, in the blockwise two-pass form); a value
 // beyond the frame, or 512 values, closes it: its count, mean and M2 become
-// doubles (frame_moments) and merge into the state.
+// doubles (frame_moments) and merge into the state.  (The frame's unit is at most
+// an eighth of its largest value's ulp, and cuts bits of values below an eighth of
+// that one only, beside which M2 is at least a third of its square: the cut moves
+// M2 by less than 2^-50 of itself.)
 template <bool W1, bool SD, class E> struct block_acc<op_moments<W1, SD>, double, E> {
   static constexpr bool value = true;
   using Op = op_moments<W1, SD>;

@@ -59,6 +59,15 @@ def test_values_no_frame_takes(gpu, cuda_lib, rows, cols, bad, at):
     assert not np.isfinite(got[1])
 
 
+@pytest.mark.parametrize("rows,cols", [(33, 70), (34, 70), (1000, 41), (10001, 7), (70, 1111), (65, 2000), (64, 2000)])
+@pytest.mark.parametrize("dim", [0, 1, 2])
+@pytest.mark.parametrize("value", [0.1, -1e16 / 3, 7e-200])
+def test_equal_values_have_no_variance(gpu, cuda_lib, rows, cols, dim, value):
+    """The frame's mean of equal values is that value, whatever pivot a ragged first trip gave."""
+    x = torch.full((rows * cols,), value, dtype=torch.float64, device="cuda")
+    assert float(api.reduce("stdev", x, rows, cols, dim=dim).abs().max()) == 0.0
+
+
 @pytest.mark.parametrize("rows", [9761, 19522])
 def test_pivot_far_from_the_values(gpu, cuda_lib, rows):
     """Rows long enough that a lane closes a frame at 512 values, whose first block (the first 64
