@@ -1035,8 +1035,9 @@ __global__ void __launch_bounds__(kStreamThreads, 1)
           sum = stream_sum{0, 0};
         }
         // lane l reads words 2 (l % 4) and the next of tile l / 4 of eight; B such
-        // loads in flight, and at most 2048 tiles before the digits are carried
-        constexpr unsigned B = kStreamLoads, STEP = 8 * kStreamGather, ROUND = 2048;
+        // loads in flight, and at most ROUND tiles before the digits are carried (a
+        // block's first gathers take several rounds, the others one)
+        constexpr unsigned B = kStreamLoads, STEP = 8 * kStreamGather, ROUND = 2 * STEP * B;
         stream_sum more{0, 0};
 #pragma unroll 1
         while (have < k) {
